@@ -185,8 +185,9 @@ ZKB_API int zkb_dft_batch_noalloc_dev(int field, void *d_rowmajor, uint32_t log_
  * loads straight into registers.  ZKB_NTT_TMA=0 in the environment selects 0 at load.
  * Results are the same bit for bit.  No counterpart in the reference. */
 ZKB_API int zkb_set_ntt_tile_loads(int mode);
-/* Tensor-copy waits of the NTT tiles that gave up (bounded polls) since the last call;
- * nonzero means those outputs are invalid.  Resets the count. */
+/* Bounded device waits that gave up since the last call: tensor copies of the NTT tiles and
+ * tensor-core products of the BabyBear hashing kernels; nonzero means those outputs are
+ * invalid.  Resets the count. */
 ZKB_API int zkb_ntt_tile_load_errors(uint32_t *count);
 
 /* p3 coset_lde_batch(trace, log_blowup, shift) followed, when bitrev_rows=1, by

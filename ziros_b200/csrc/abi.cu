@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "engine.cuh"
+#include "p2_launch.cuh"
 
 namespace zkb {
 const char *last_error();
@@ -274,7 +275,11 @@ int zkb_set_ntt_tile_loads(int mode) {
 int zkb_ntt_tile_load_errors(uint32_t *count) {
   ZKB_ENTRY();
   ZKB_REQUIRE(count != nullptr, "null count");
-  return ntt_tma_wait_errors(count);
+  uint32_t hashing = 0;
+  ZKB_TRY(p2t::wait_errors(&hashing));
+  ZKB_TRY(ntt_tma_wait_errors(count));
+  *count += hashing;
+  return ZKB_OK;
 }
 
 int zkb_dft_batch(int field, void *rowmajor, uint32_t log_h, uint32_t width, int inverse) {

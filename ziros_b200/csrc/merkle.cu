@@ -17,30 +17,15 @@
 
 #include "common.cuh"
 #include "engine.cuh"
+#include "matlist.cuh"
+#include "p2_launch.cuh"
 #include "poseidon2.cuh"
 
 namespace zkb {
 
-constexpr int MAX_GROUP_MATS = 16;
-
-struct MatList {
-  const void *ptr[MAX_GROUP_MATS];
-  uint64_t width[MAX_GROUP_MATS];
-  uint64_t col_start[MAX_GROUP_MATS + 1];
-  int n;
-};
-
 template <int W>
 __host__ __device__ constexpr int p2_out() {
   return W == 16 ? 8 : 4;
-}
-
-template <class F>
-__device__ __forceinline__ typename F::T fetch_col(const MatList &ml, uint64_t row, uint64_t col) {
-  int m = 0;
-  while (m + 1 < ml.n && col >= ml.col_start[m + 1]) m++;
-  const typename F::T *base = (const typename F::T *)ml.ptr[m];
-  return base[row * ml.width[m] + (col - ml.col_start[m])];
 }
 
 // Leaf digests: PaddingFreeSponge over the concatenated row of the matrices in ml.
@@ -337,8 +322,10 @@ static int build_tree_impl(const HasherSpec &h, const std::vector<TreeMatrix> &m
     ZKB_REQUIRE(nm == 1 && comb == nullptr, "internal: leaves written by the caller take one matrix");
     ZKB_TRY((*fill)(layers));
   } else if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
-    if (comb) {
-      ZKB_REQUIRE(nm == 1, "the fused alpha-reduction takes one matrix");
+    if (comb) ZKB_REQUIRE(nm == 1, "the fused alpha-reduction takes one matrix");
+    if (ml.col_start[ml.n] > 0 && p2t::takes(p, max_h)) {
+      ZKB_TRY(p2t::hash_rows(ml, max_h, layers, p, comb ? comb->apow : nullptr, comb ? comb->out : nullptr, leaf_name, s));
+    } else if (comb) {
       ZKB_LAUNCH(leaf_name, s, hash_rows_combine_kernel<<<grid_for(max_h, thr, cap), thr, 0, s>>>((const uint32_t *)ml.ptr[0], ml.width[0], max_h, layers, p, comb->apow, comb->out));
     } else {
       ZKB_LAUNCH(leaf_name, s, hash_rows_kernel<F, W><<<grid_for(max_h, thr, cap), thr, 0, s>>>(ml, max_h, layers, p));
@@ -366,13 +353,23 @@ static int build_tree_impl(const HasherSpec &h, const std::vector<TreeMatrix> &m
       ZKB_TRY(make_list(next_m, ni, &iml));
       inj_h = mats[ord[next_m]].height;
       if (!inj_buf.p) ZKB_TRY(inj_buf.alloc(inj_h * OUT * sizeof(T), s));
-      ZKB_LAUNCH("merkle_inject_hash", s, hash_rows_kernel<F, W><<<grid_for(inj_h, thr, cap), thr, 0, s>>>(iml, inj_h, inj_buf.as<T>(), p));
-      ZKB_CHECK_LAUNCH();
+      bool tensor = false;
+      if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
+        tensor = iml.col_start[iml.n] > 0 && p2t::takes(p, inj_h);
+        if (tensor) ZKB_TRY(p2t::hash_rows(iml, inj_h, inj_buf.as<T>(), p, nullptr, nullptr, "merkle_inject_hash", s));
+      }
+      if (!tensor)
+        ZKB_LAUNCH("merkle_inject_hash", s, hash_rows_kernel<F, W><<<grid_for(inj_h, thr, cap), thr, 0, s>>>(iml, inj_h, inj_buf.as<T>(), p));
       inj = inj_buf.as<T>();
     }
     next_m += ni;
+    if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
+      if (p2t::takes(p, half)) {
+        ZKB_TRY(p2t::compress(prev, next, half, inj, inj_h, p, comp_name, s));
+        continue;
+      }
+    }
     ZKB_LAUNCH(comp_name, s, compress_kernel<F, W><<<grid_for(half, thr, cap), thr, 0, s>>>(prev, next, half, inj, inj_h, p));
-    ZKB_CHECK_LAUNCH();
   }
   return ZKB_OK;
 }
@@ -391,14 +388,18 @@ int hash_rows_slab_dev(const HasherSpec &h, const uint32_t *mat, uint64_t stride
                        uint64_t height, uint32_t *carry, bool first, bool last, uint32_t *digests,
                        const LeafCombine *comb, cudaStream_t s) {
   ZKB_REQUIRE(h.field == FIELD_BABYBEAR && h.width == 16, "internal: slab leaf hashing is BabyBear width 16");
-  ZKB_REQUIRE(c0 % 8 == 0 && (last || ncols % 8 == 0), "internal: slabs hold whole absorbed chunks");
+  ZKB_REQUIRE(ncols > 0 && c0 % 8 == 0 && (last || ncols % 8 == 0), "internal: slabs hold whole absorbed chunks");
   P2Params<BabyBear, 16> p;
   if (!build_p2_params<BabyBear, 16>(h, &p)) {
     set_error("invalid Poseidon2 parameters");
     return ZKB_ERR_INVALID;
   }
+  const uint4 *apow = comb ? comb->apow : nullptr;
+  uint4 *out = comb ? comb->out : nullptr;
+  if (p2t::takes(p, height))  // by the height alone: every slab of a matrix takes the same form
+    return p2t::hash_slab(mat, stride, c0, ncols, height, carry, first, last, digests, p, apow, out, "merkle_leaf_hash", s);
   const unsigned thr = 128;
-  ZKB_LAUNCH("merkle_leaf_hash", s, hash_rows_slab_kernel<<<grid_for(height, thr, 1u << 30), thr, 0, s>>>(mat, stride, c0, ncols, height, carry, first ? 1 : 0, last ? 1 : 0, digests, p, comb ? comb->apow : nullptr, comb ? comb->out : nullptr));
+  ZKB_LAUNCH("merkle_leaf_hash", s, hash_rows_slab_kernel<<<grid_for(height, thr, 1u << 30), thr, 0, s>>>(mat, stride, c0, ncols, height, carry, first ? 1 : 0, last ? 1 : 0, digests, p, apow, out));
   return ZKB_OK;
 }
 

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "p2_launch.cuh"
 #include "poseidon2.cuh"
 
 namespace zkb {
@@ -22,6 +23,7 @@ struct LeafJob {
   uint64_t row_start;  // prefix over the jobs
   uint64_t rows;
   uint64_t width;
+  uint64_t tile_start;  // prefix over the jobs in 128-row tiles (no tile spans two jobs)
 };
 
 struct CompJob {
@@ -135,6 +137,9 @@ struct Tables {
   std::vector<uint64_t> root_off;
   std::vector<std::vector<uint64_t>> layer_len;
   uint64_t total_rows = 0;
+  uint64_t tiles = 0;      // 128-row tiles
+  uint64_t max_perms = 0;  // permutations of the widest row
+  bool empty_rows = false;
 
   // device bytes of the tables (leaf jobs, compression jobs, root offsets)
   uint64_t device_bytes() const {
@@ -152,8 +157,11 @@ inline void build_tables(const std::vector<const void *> &data, const std::vecto
   t->layer_len.assign(n, {});
   size_t max_levels = 0;
   for (size_t i = 0; i < n; i++) {
-    t->leaf[i] = LeafJob{data[i], layers[i], t->total_rows, rows[i], width[i]};
+    t->leaf[i] = LeafJob{data[i], layers[i], t->total_rows, rows[i], width[i], t->tiles};
     t->total_rows += rows[i];
+    t->tiles += (rows[i] + 127) / 128;
+    t->max_perms = std::max(t->max_perms, (width[i] + 7) / 8);
+    t->empty_rows = t->empty_rows || width[i] == 0;
     uint64_t o = 0;
     for (uint64_t len = rows[i];; len /= 2) {
       t->layer_len[i].push_back(len);
@@ -214,9 +222,25 @@ int launch_trees(const Tables &t, const LeafJob *d_leaf, const CompJob *d_comp, 
   // one row (or compression) per thread: short-lived blocks, so concurrent streams
   // interleave at block granularity
   (void)ctx;
-  if (leaf_name)
+  constexpr bool bb16 = std::is_same<F, BabyBear>::value && W == 16;
+  bool leaves_done = leaf_name == nullptr;
+  if constexpr (bb16) {
+    // Tiles hold 128 rows of one job: jobs of fewer rows leave lanes idle, and with more than a
+    // quarter of the lanes idle the row-per-thread kernel is the faster one.
+    if (!leaves_done && !t.empty_rows && p2t::takes(p, t.total_rows) && t.tiles * 128 <= t.total_rows + t.total_rows / 4) {
+      ZKB_TRY(p2t::mt_leaf(d_leaf, n, t.tiles, t.max_perms, p, leaf_name, s));
+      leaves_done = true;
+    }
+  }
+  if (!leaves_done)
     ZKB_LAUNCH(leaf_name, s, mt_leaf_kernel<F, W><<<grid_for(t.total_rows, leaf_threads, 1u << 30), leaf_threads, n * sizeof(uint64_t), s>>>(d_leaf, n, t.total_rows, p));
   for (size_t l = 0; l < t.lvl_cnt.size(); l++) {
+    if constexpr (bb16) {
+      if (p2t::takes(p, t.lvl_total[l])) {
+        ZKB_TRY(p2t::mt_compress(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p, comp_name, s));
+        continue;
+      }
+    }
     ZKB_LAUNCH(comp_name, s, mt_compress_kernel<F, W><<<grid_for(t.lvl_total[l], 128, 1u << 30), 128, t.lvl_cnt[l] * sizeof(uint64_t), s>>>(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p));
   }
   ZKB_LAUNCH(root_name, s, mt_roots_kernel<T, OUT><<<(n * OUT + 127) / 128, 128, 0, s>>>(d_root_off, (const T *)base, n, d_root_dst, (T *)d_roots));

@@ -1,0 +1,42 @@
+// p2_launch.cuh — launches of the tensor-core hashing kernels (p2_tensor.cu).
+#pragma once
+#include "common.cuh"
+#include "fri_fold.cuh"
+#include "matlist.cuh"
+#include "poseidon2.cuh"
+
+namespace zkb {
+namespace mt {
+struct LeafJob;
+struct CompJob;
+}  // namespace mt
+
+namespace p2t {
+
+// True when a launch over this many rows (or compressions) takes the tensor-core kernels.
+bool takes(const P2Params<BabyBear, 16> &p, uint64_t rows);
+// Leaf digests of `height` rows (total width at least 1); with comb (one matrix) the rows'
+// alpha-reductions too.
+int hash_rows(const MatList &ml, uint64_t height, uint32_t *digests, const P2Params<BabyBear, 16> &p,
+              const uint4 *apow, uint4 *comb, const char *name, cudaStream_t s);
+// A slab of columns; every slab of a matrix goes through the same form (the carried words differ).
+int hash_slab(const uint32_t *mat, uint64_t stride, uint64_t c0, uint64_t ncols, uint64_t height, uint32_t *carry,
+              bool first, bool last, uint32_t *digests, const P2Params<BabyBear, 16> &p, const uint4 *apow, uint4 *comb,
+              const char *name, cudaStream_t s);
+int compress(const uint32_t *prev, uint32_t *next, uint64_t n_out, const uint32_t *inj, uint64_t inj_h,
+             const P2Params<BabyBear, 16> &p, const char *name, cudaStream_t s);
+// Leaves of many matrices: `tiles` 128-row tiles (LeafJob::tile_start), `perms` the largest
+// row's permutations.
+int mt_leaf(const mt::LeafJob *d_jobs, int n, uint64_t tiles, uint64_t perms, const P2Params<BabyBear, 16> &p,
+            const char *name, cudaStream_t s);
+int mt_compress(const mt::CompJob *d_jobs, int n, uint64_t total, const P2Params<BabyBear, 16> &p, const char *name,
+                cudaStream_t s);
+int fri_fold_hash(const uint32_t *e, uint32_t *out, uint64_t n_leaves, int log_out, const Ext4Params *prm,
+                  const uint32_t *itw, uint32_t *digests, const P2Params<BabyBear, 16> &p, const char *name,
+                  cudaStream_t s);
+int permute(uint32_t *states, uint64_t n, const P2Params<BabyBear, 16> &p, cudaStream_t s);
+// Waits that gave up since the last call (resets the count).
+int wait_errors(uint32_t *count);
+
+}  // namespace p2t
+}  // namespace zkb

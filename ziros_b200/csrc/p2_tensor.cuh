@@ -1,0 +1,685 @@
+// p2_tensor.cuh — BabyBear width-16 Poseidon2 with its linear layers on the tensor cores.
+//
+// The permutation's linear layers are 16 x 16 matrices over F_p and its S-boxes are
+// element-wise, so the layers run as integer matrix products on the tensor cores
+// (tcgen05.mma kind::i8, 128 x N x 32 steps, exact s32 accumulation in TMEM) while the
+// integer pipes do the S-boxes.  One thread owns one permutation, and a group of 128
+// threads (four warps, the 128 TMEM lanes) shares one product per layer:
+//   A (TMEM): row = thread; the thread's u32 words, written by tcgen05.st.  The four bytes of a
+//      word ARE four consecutive 8-bit operands, so no limb is ever split off.
+//   B (shared memory): the layer's matrix.  Entry c of the layer, against byte l' of an input
+//      word, contributes c * 2^(8 l') mod p; byte l of that constant goes to column (output, l).
+//      (A small entry c <= 255 simply puts c in column (output, l').)
+//   D (TMEM): four s32 accumulators per output word, weights 2^0, 2^8, 2^16, 2^24.
+// A thread reads its accumulators back (tcgen05.ld), recombines each output with six integer
+// operations and a Barrett quotient instead of the additions mod p of the layer, and goes on with
+// the next S-box.  Round constants ride on a constant-one operand byte.  The thirteen
+// partial rounds have one S-box each and are linear otherwise: the S-box inputs y_k are
+// functionals of the state that entered them plus known multiples of the S-box outputs
+// w_j (j < k), so three products (blocks of 4, 4 and 5 rounds) and a few scalar products
+// replace thirteen dense rounds.  The last layer of a permutation and the first layer of the
+// next absorb step are one product.
+#pragma once
+#include "field.cuh"
+#include "poseidon2.cuh"
+
+namespace zkb {
+namespace p2t {
+
+constexpr int NF = 8, NP = 13;   // rounds this form is built for (R_F, R_P)
+constexpr int GROUP = 128;       // threads (= permutations) of one product
+constexpr int MAX_GROUPS = 5;    // per block: 5 * 96 columns <= 512
+constexpr int COLS = 96;         // TMEM columns of a group: D 64, Z 16, W 16
+constexpr int COL_D = 0, COL_Z = 64, COL_W = 80;
+constexpr int W_ONE = 13;        // word of the W region holding the constant 1
+constexpr uint32_t P = BabyBear::P;
+constexpr uint32_t SMALL_BIAS = 0x4B400000u;  // see recombine_small
+
+// ------------------------------------------------------------- coefficients (host)
+// Each coefficient is stored as its four limb multiples c * 2^(8 l) mod p.
+struct Coefs {
+  uint32_t in[16][16][4];    // M * R: canonical input word -> state (Montgomery)
+  uint32_t y[13][16][4];     // state that entered the last initial full round's layer -> y_k
+  uint32_t oz[16][16][4];    // ... -> state after the partial rounds
+  uint32_t ow[16][13][4];    // w_j -> state after the partial rounds
+  uint32_t c[13][4];         // y_k += c[k-1-j] * w_j
+  uint32_t fin[16][16][4];   // M * R^-1: last S-box outputs -> canonical state
+  uint32_t cm[13];           // c[i] as the centred Montgomery multiplier of a scalar product, negated
+  uint8_t m[16][16];         // external matrix
+};
+
+constexpr uint32_t mulp(uint32_t a, uint32_t b) { return (uint32_t)((uint64_t)a * b % P); }
+constexpr uint32_t addp(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a + b) % P); }
+constexpr uint32_t powp(uint32_t a, uint32_t e) {
+  uint32_t r = 1;
+  while (e) {
+    if (e & 1) r = mulp(r, a);
+    a = mulp(a, a);
+    e >>= 1;
+  }
+  return r;
+}
+constexpr void limbs(uint32_t (&o)[4], uint32_t c) {
+  for (int l = 0; l < 4; l++) {
+    o[l] = c;
+    c = mulp(c, 256);
+  }
+}
+
+constexpr Coefs make_coefs() {
+  Coefs k{};
+  const uint32_t R = (uint32_t)((1ull << 32) % P), Ri = powp(R, P - 2);
+  const uint8_t m4[4][4] = {{2, 3, 1, 1}, {1, 2, 3, 1}, {1, 1, 2, 3}, {3, 1, 1, 2}};
+  for (int i = 0; i < 16; i++)
+    for (int j = 0; j < 16; j++) k.m[i][j] = (uint8_t)(m4[i % 4][j % 4] * (i / 4 == j / 4 ? 2 : 1));
+  // internal diagonal V (poseidon2.cuh: bb16::internal_round)
+  const uint32_t i2 = powp(2, P - 2), i8 = powp(256, P - 2), i27 = powp(1u << 27, P - 2);
+  const uint32_t d[16] = {P - 2, 1, 2, i2, 3, 4, P - i2, P - 3, P - 4, i8, mulp(i2, i2), mulp(i2, mulp(i2, i2)),
+                          i27, P - i8, P - powp(16, P - 2), P - i27};
+  // a = A e0, Abar = A with column 0 cleared; Abar v = d_i v_i + sum_{j>=1} v_j (lane 0 in: 0)
+  uint32_t a[16] = {};
+  for (int i = 0; i < 16; i++) a[i] = i == 0 ? addp(d[0], 1) : 1;
+  // functionals f_k = e0^T Abar^k M and c_k = e0^T Abar^k a
+  uint32_t f[16] = {};
+  f[0] = 1;
+  for (int t = 0; t < 13; t++) {
+    for (int j = 0; j < 16; j++) {
+      uint32_t s = 0;
+      for (int i = 0; i < 16; i++) s = addp(s, mulp(f[i], k.m[i][j]));
+      limbs(k.y[t][j], s);
+    }
+    uint32_t c = 0;
+    for (int i = 0; i < 16; i++) c = addp(c, mulp(f[i], a[i]));
+    limbs(k.c[t], c);
+    const uint32_t neg = mulp(c ? P - c : 0, R);
+    k.cm[t] = neg > P / 2 ? neg - P : neg;  // centred (two's complement)
+    uint32_t sum = 0;
+    for (int i = 0; i < 16; i++) sum = addp(sum, f[i]);
+    uint32_t g[16] = {};
+    for (int j = 1; j < 16; j++) g[j] = addp(sum, mulp(d[j], f[j]));
+    for (int j = 0; j < 16; j++) f[j] = g[j];
+  }
+  // columns after the partial rounds
+  for (int j = 0; j < 16 + 13; j++) {
+    uint32_t v[16] = {};
+    int steps = 13;
+    if (j < 16) {
+      for (int i = 0; i < 16; i++) v[i] = k.m[i][j];
+    } else {
+      for (int i = 0; i < 16; i++) v[i] = a[i];
+      steps = 12 - (j - 16);
+    }
+    for (int t = 0; t < steps; t++) {
+      uint32_t sum = 0;
+      for (int i = 1; i < 16; i++) sum = addp(sum, v[i]);
+      for (int i = 1; i < 16; i++) v[i] = addp(sum, mulp(d[i], v[i]));
+      v[0] = sum;
+    }
+    // the next full round adds its constants and applies x^7 to this state directly
+    for (int i = 0; i < 16; i++) {
+      if (j < 16)
+        limbs(k.oz[i][j], v[i]);
+      else
+        limbs(k.ow[i][j - 16], v[i]);
+    }
+  }
+  for (int i = 0; i < 16; i++)
+    for (int j = 0; j < 16; j++) {
+      limbs(k.in[i][j], mulp(k.m[i][j], R));
+      limbs(k.fin[i][j], mulp(k.m[i][j], Ri));
+    }
+  return k;
+}
+
+// True when these parameters are the instance the tables above describe.
+inline bool usable(const P2Params<BabyBear, 16> &p) {
+  return p.diag_kind == 1 && p.rounds_f == NF && p.rounds_p == NP;
+}
+
+
+// ------------------------------------------------------------------ layer matrices
+// A slab is one 32-byte K step: N rows x 32 bytes in 8 x 16-byte core matrices,
+// [k / 16][n / 8][n % 8][k % 16].  Image offsets (bytes); the first five are copied as they lie.
+constexpr int SLAB64 = 2048;
+constexpr int I_EXT = 0;                      // M against Z: 2 slabs
+constexpr int I_Y = I_EXT + 2 * SLAB64;       // 2 slabs
+constexpr int I_O = I_Y + 2 * SLAB64;         // Z 2 slabs, W 2
+constexpr int I_B2 = I_O + 4 * SLAB64;        // N = 48
+constexpr int I_B3 = I_B2 + 48 * 32;          // N = 32
+constexpr int COMMON = I_B3 + 32 * 32;
+constexpr int I_FIN8 = COMMON;                // N = 32: 2 slabs of 1024
+constexpr int I_FIN16 = I_FIN8 + SLAB64;      // N = 64: 2 slabs
+constexpr int I_IN16 = I_FIN16 + 2 * SLAB64;  // 16 canonical words in: 2 slabs
+constexpr int I_ABS = I_IN16 + 2 * SLAB64;    // absorb chunks of 8, 1, 2, ... 7 words: Z 2 slabs, input 1
+constexpr int ABS_BYTES = 3 * SLAB64;
+constexpr int IMAGE = I_ABS + 8 * ABS_BYTES;
+
+// Column of an output's weight-2^(8 l) accumulator among its four: 0, 2, 1, 3, so that the low
+// halves of adjacent columns pack into a0 + a2 2^16 and a1 + a3 2^16.
+__host__ __device__ constexpr int acc_col(int l) { return l == 1 ? 2 : l == 2 ? 1 : l; }
+__host__ __device__ constexpr int slot(int N, int n, int k) {
+  return ((k >> 4) * (N >> 3) + (n >> 3)) * 128 + (n & 7) * 16 + (k & 15);
+}
+
+struct alignas(16) Image {
+  uint8_t b[IMAGE];
+  constexpr void gen(int base, int N, int i, int j, const uint32_t (&c)[4]) {
+    for (int lp = 0; lp < 4; lp++)
+      for (int l = 0; l < 4; l++) b[base + slot(N, 4 * i + acc_col(l), 4 * j + lp)] = (uint8_t)(c[lp] >> (8 * l));
+  }
+  constexpr void small(int base, int N, int i, int j, uint32_t c) {
+    for (int l = 0; l < 4; l++) b[base + slot(N, 4 * i + acc_col(l), 4 * j + l)] = (uint8_t)c;
+  }
+};
+
+constexpr Image make_image() {
+  Image m{};
+  const Coefs k = make_coefs();
+  for (int i = 0; i < 16; i++)
+    for (int j = 0; j < 16; j++) {
+      m.small(I_EXT, 64, i, j, k.m[i][j]);
+      m.gen(I_O, 64, i, j, k.oz[i][j]);
+      if (i < 13) m.gen(I_Y, 64, i, j, k.y[i][j]);
+      if (j < 13) m.gen(I_O + 2 * SLAB64, 64, i, j, k.ow[i][j]);
+      if (i < 8) m.gen(I_FIN8, 32, i, j, k.fin[i][j]);
+      m.gen(I_FIN16, 64, i, j, k.fin[i][j]);
+      m.gen(I_IN16, 64, i, j, k.in[i][j]);
+      // y_k += c[k-1-j] w_j: block 2 (j 0..3 -> k 4..12) and block 3 (j 4..7 -> k 8..12)
+      if (i < 9 && j < 4) m.gen(I_B2, 48, i, j, k.c[i + 3 - j]);
+      if (i < 5 && j >= 4 && j < 8) m.gen(I_B3, 32, i, j, k.c[i + 7 - j]);
+    }
+  // Absorbing `rem` words: lane l < rem takes its input word, the others keep the last
+  // permutation's state M z; the first layer of the next is M again.
+  for (int rem = 1; rem <= 8; rem++) {
+    const int base = I_ABS + (rem % 8) * ABS_BYTES;
+    for (int i = 0; i < 16; i++) {
+      for (int j = 0; j < 16; j++) {
+        uint32_t s = 0;
+        for (int l = rem; l < 16; l++) s += (uint32_t)k.m[i][l] * k.m[l][j];
+        m.small(base, 64, i, j, s);  // at most 255: checked below
+      }
+      for (int j = 0; j < rem; j++) m.gen(base + 2 * SLAB64, 64, i, j, k.in[i][j]);
+    }
+  }
+  return m;
+}
+constexpr bool absorb_fits() {
+  const Coefs k = make_coefs();
+  for (int i = 0; i < 16; i++)
+    for (int j = 0; j < 16; j++) {
+      int s = 0;
+      for (int l = 1; l < 16; l++) s += k.m[i][l] * k.m[l][j];
+      if (s > 255) return false;
+    }
+  return true;
+}
+static_assert(absorb_fits(), "the fused absorb layer needs entries below 256");
+
+#ifdef __CUDACC__
+static __device__ constexpr Coefs kCoefs = make_coefs();
+static __device__ const Image kImage = make_image();
+
+// ------------------------------------------------------------------- shared memory
+enum Mode { SPONGE = 0, SPONGE_ANY = 1, STATE16 = 2, PERM16 = 3 };
+constexpr int S_C = COMMON;                  // constants: first layer, rounds 1-3, y, terminal 1-3
+constexpr int S_FIN = S_C + 8 * SLAB64;      // last layer: 2 slabs of N = 32, or of N = 64 (PERM16)
+constexpr int S_IN = S_FIN + 2 * SLAB64;     // 16-word input (2 slabs), or absorb matrices: full chunk,
+                                             // then the partial one (SPONGE) or those of 1..7 words (SPONGE_ANY)
+constexpr int S_LAST = S_IN + ABS_BYTES;
+__host__ __device__ constexpr int smem_tables(Mode m) {
+  return m == SPONGE ? S_LAST + ABS_BYTES : m == SPONGE_ANY ? S_LAST + 7 * ABS_BYTES : S_IN + 2 * SLAB64;
+}
+// TMEM address, the image's mbarrier and one per group follow the tables.
+__host__ __device__ constexpr int smem_bytes(Mode m) { return smem_tables(m) + 16 + 8 * MAX_GROUPS; }
+
+// A part of the image, copied by one untiled bulk copy of this GPU's own memory.
+__device__ __forceinline__ void copy_tables(uint32_t dst, int src, int bytes, uint32_t mbar) {
+  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(__cvta_generic_to_global(kImage.b + src)), "r"((uint32_t)bytes), "r"(mbar)
+               : "memory");
+}
+// The matrices a kernel needs: issued by one thread, completed on mbar.
+__device__ __forceinline__ void copy_image(uint32_t sm, Mode mode, int last_rem, uint32_t mbar) {
+  const bool sponge = mode == SPONGE || mode == SPONGE_ANY;
+  const int fin = mode == PERM16 ? 2 * SLAB64 : SLAB64, in = sponge ? ABS_BYTES : 2 * SLAB64;
+  const int last = mode == SPONGE_ANY ? 7 * ABS_BYTES : mode == SPONGE && last_rem != 8 ? ABS_BYTES : 0;
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar),
+               "r"((uint32_t)(COMMON + fin + in + last))
+               : "memory");
+  copy_tables(sm, 0, COMMON, mbar);
+  copy_tables(sm + S_FIN, mode == PERM16 ? I_FIN16 : I_FIN8, fin, mbar);
+  copy_tables(sm + S_IN, sponge ? I_ABS : I_IN16, in, mbar);
+  if (last) copy_tables(sm + S_LAST, I_ABS + (mode == SPONGE_ANY ? 1 : last_rem) * ABS_BYTES, last, mbar);
+}
+// The round constants: byte 4 * (W_ONE - 8) of the second W slab meets the constant one.
+__device__ __forceinline__ void put_constants(uint8_t *sm, const P2Params<BabyBear, 16> &p) {
+  constexpr int kb = 4 * (W_ONE - 8);
+  for (int t = threadIdx.x; t < 9 * 16; t += blockDim.x) {
+    const int r = t >> 4, i = t & 15;
+    uint32_t v;
+    int base = S_C + r * SLAB64;
+    if (r < 4)
+      v = p.rc[r * 16 + i] + (r ? SMALL_BIAS : 0);  // first layer, rounds 1..3
+    else if (r == 4)
+      v = i < NP ? p.rc[64 + i] : 0;
+    else {
+      v = p.rc[64 + NP + (r - 5) * 16 + i] + (r > 5 ? SMALL_BIAS : 0);  // terminal rounds 0..3
+      base = r == 5 ? I_O + 3 * SLAB64 : S_C + (r - 1) * SLAB64;
+    }
+#pragma unroll
+    for (int l = 0; l < 4; l++) sm[base + slot(64, 4 * i + acc_col(l), kb)] = (uint8_t)(v >> (8 * l));
+  }
+}
+
+// ------------------------------------------------------------------- PTX wrappers
+// s32 accumulators, u8 x u8, both operands K-major, M = 128.
+__device__ __forceinline__ constexpr uint32_t idesc(int N) {
+  return (2u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(GROUP >> 4) << 24);
+}
+// Shared-memory operand without swizzle: 8 x 16-byte core matrices, 128 bytes apart along N and
+// (N / 8) * 128 bytes apart along K.
+__device__ __forceinline__ uint64_t bdesc(uint32_t addr, int N) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((N / 8) * 128 / 16) << 16) | ((uint64_t)(128 / 16) << 32) |
+         (1ull << 46);
+}
+// Issued by a whole warp with warp-uniform operands; `one` is set in a single lane.
+__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint64_t b, uint32_t id, bool acc, uint32_t one) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\tsetp.ne.u32 p, %4, 0;\n\tsetp.ne.u32 e, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+      "r"(a), "l"(b), "r"(id), "r"((uint32_t)acc), "r"(one)
+      : "memory");
+}
+__device__ __forceinline__ void st8(uint32_t a, const uint32_t *v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(a), "r"(v[0]), "r"(v[1]),
+               "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+__device__ __forceinline__ void st4(uint32_t a, const uint32_t *v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3])
+               : "memory");
+}
+__device__ __forceinline__ void st1(uint32_t a, uint32_t v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void ld16(uint32_t (&v)[16], uint32_t a) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(a)
+      : "memory");
+}
+// The low 16 bits of 32 columns, two adjacent columns to a register.
+__device__ __forceinline__ void ld16_pack(uint32_t (&v)[16], uint32_t a) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(a)
+      : "memory");
+}
+// Waits for the loads; the registers pass through so that no use moves above the wait.
+__device__ __forceinline__ void ld_wait(uint32_t (&v)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
+}
+
+// --------------------------------------------------------------------- arithmetic
+// Signed Montgomery product: any int32 operands (the result, hi(a b) - hi(m p), lies in
+// (-2^31, 2^31), and in (-p, p) for |a b| < 2^31 p).  Five multiplier issue slots: a wide
+// product, a low one, a high one.
+__device__ __forceinline__ int smul(int a, int b) {
+  const int64_t t = (int64_t)a * b;
+  const int m = (int)((uint32_t)t * BabyBear::PINV);
+  return (int)(t >> 32) - __mulhi(m, (int)P);
+}
+__device__ __forceinline__ int smul2(int a0, int b0, int a1, int b1) {
+  const int64_t t = (int64_t)a0 * b0 + (int64_t)a1 * b1;
+  const int m = (int)((uint32_t)t * BabyBear::PINV);
+  return (int)(t >> 32) - __mulhi(m, (int)P);
+}
+// x^7 of any int32 input, in (-p, p): |x2| <= 2^30 + p/2, |x3| <= 2^30 + p/2, |x4| < p, so the last
+// product has |x3 x4| < 2^62 / 2.
+__device__ __forceinline__ int sbox(int x) {
+  const int x2 = smul(x, x);
+  const int x3 = smul(x2, x);
+  const int x4 = smul(x2, x2);
+  return smul(x3, x4);
+}
+// [-p, p) -> [0, p); also [-p, 1.06 p] -> [0, 1.06 p]
+__device__ __forceinline__ uint32_t lift(int x) {
+  const uint32_t a = (uint32_t)x, b = a + P;
+  return a < b ? a : b;
+}
+// The output word of four accumulators, congruent to a0 + a1 2^8 + a2 2^16 + a3 2^24 mod p and in
+// [-p, 1.04 p]: u = a0 + a1 2^8 and v = a2 + a3 2^8 stay below 0.97 p (at most 120 operand
+// bytes, 120 * 255 * 255 * 257 < 2^31); q = floor(v * 139810 / 2^32) is at most the true quotient of
+// v 2^16 by p (2^32 * 2^16 / p = 139810.13) and less than 1.07 below it.
+__device__ __forceinline__ int recombine(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+  const uint32_t u = a0 + (a1 << 8), v = a2 + (a3 << 8);
+  const uint32_t q = __umulhi(v, 139810u) + 1;
+  return (int)(u + (v << 16) - q * P);
+}
+// The same for the external matrix alone, whose accumulators stay below 2^14 (35 * 255 + 255), read
+// in pairs as p02 = a0 + a2 2^16 and p13 = a1 + a3 2^16.  The quotient comes from a3 as a float:
+// f = 2^15 + a3 exactly, k = (1 - 0.00146) 2^24 / p, so f k - 273 lies between 0.33 and 0.45 below
+// a3 2^24 / p and the fma rounds it to q in the low mantissa bits, 0x4B400000 + q.  The rest of the
+// accumulators is worth at most 0.3 p, so t - q p lies in [-0.17 p, 1.25 p]; the 0x4B400000 p that
+// is subtracted with it equals 0x4B400000 mod 2^32 (0.627 p), which the round constants carry
+// (SMALL_BIAS), leaving [-0.8 p, 0.63 p].
+__device__ __forceinline__ int recombine_small(uint32_t p02, uint32_t p13) {
+  const uint32_t t = p02 + (p13 << 8);
+  const float f = __uint_as_float(__byte_perm(p13, 0x47000000u, 0x7324));
+  const float k = (float)(16777216.0 / 2013265921.0 * (1.0 - 0.00146));
+  const float q = __fmaf_rn(f, k, 12582912.0f - 273.0f);
+  return (int)(t - __float_as_uint(q) * P);
+}
+
+// ------------------------------------------------------------------------- a group
+struct Group {
+  uint32_t sm;      // shared address of the tables
+  uint32_t tm;      // TMEM address of the group's columns
+  uint32_t tw;      // the same with this warp's lane base (ld / st)
+  uint32_t mbar;    // shared address of the group's mbarrier
+  uint32_t phase;
+  int bar;          // named barrier of the group
+  bool lead;        // this is the warp that issues the products (warp-uniform)
+  uint32_t one;     // set in one lane of it
+  uint32_t polls;   // limit of a wait (0 once one has run out)
+  uint32_t *err;
+};
+
+constexpr uint32_t WAIT_POLLS = 1u << 16;
+
+__device__ __forceinline__ void mma_slab(const Group &g, int d_col, int a_col, int off, int N, bool acc) {
+  mma(g.tm + d_col, g.tm + a_col, bdesc(g.sm + off, N), idesc(N), acc, g.one);
+}
+
+__device__ __forceinline__ bool wait_parity(uint32_t mbar, uint32_t parity, uint32_t polls) {
+  uint32_t done = 0;
+  for (uint32_t n = 0; n < polls && !done; n++) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+  }
+  return done != 0;
+}
+
+// Before the products: this thread's operand stores are complete and its accumulator loads done.
+__device__ __forceinline__ void arrive(const Group &g) {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  asm volatile("bar.sync %0, 128;" ::"r"(g.bar) : "memory");
+  if (g.lead) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+// After the products have been issued by the lead thread: everyone waits for them (bounded: a
+// wait that runs out records itself and the group goes on, so every block ends).
+__device__ __forceinline__ void finish(Group &g) {
+  if (g.lead)
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.u32 e, %1, 0;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(g.mbar),
+        "r"(g.one)
+        : "memory");
+  if (!wait_parity(g.mbar, g.phase, g.polls)) {
+    if (g.polls) atomicAdd(g.err, 1u);
+    g.polls = 0;
+  }
+  g.phase ^= 1;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+
+// One layer's outputs to S-box outputs: 16 words, each x^7 + p in (0, 2p), stored as the next
+// operand.
+template <bool SMALL>
+__device__ __forceinline__ void full_sbox(const Group &g) {
+  uint32_t z[16];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    if constexpr (SMALL) {
+      uint32_t a[16];
+      ld16_pack(a, g.tw + COL_D + 32 * h);
+      ld_wait(a);
+#pragma unroll
+      for (int e = 0; e < 8; e++) z[8 * h + e] = (uint32_t)sbox(recombine_small(a[2 * e], a[2 * e + 1])) + P;
+    } else {
+      uint32_t a[16], b[16];
+      ld16(a, g.tw + COL_D + 32 * h);
+      ld16(b, g.tw + COL_D + 32 * h + 16);
+      ld_wait(a);
+      ld_wait(b);
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        z[8 * h + e] = (uint32_t)sbox(recombine(a[4 * e], a[4 * e + 2], a[4 * e + 1], a[4 * e + 3])) + P;
+        z[8 * h + 4 + e] = (uint32_t)sbox(recombine(b[4 * e], b[4 * e + 2], b[4 * e + 1], b[4 * e + 3])) + P;
+      }
+    }
+  }
+  st8(g.tw + COL_Z, z);
+  st8(g.tw + COL_Z + 8, z + 8);
+}
+
+// y_k of a block of partial rounds starting at k0: base (its accumulators) plus the known
+// multiples of the block's earlier w: c_0 = -1 exactly, the others as scalar products.
+template <int K0, int CNT>
+__device__ __forceinline__ void partial_block(const Group &g, int (&w)[13]) {
+  int b[CNT];
+  {
+    uint32_t a[16];
+    ld16(a, g.tw + COL_D + 4 * K0);
+    ld_wait(a);
+#pragma unroll
+    for (int e = 0; e < 4; e++) b[e] = recombine(a[4 * e], a[4 * e + 2], a[4 * e + 1], a[4 * e + 3]);
+  }
+  if constexpr (CNT == 5) {
+    uint32_t a[4];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+                 : "r"(g.tw + COL_D + 4 * (K0 + 4))
+                 : "memory");
+    b[4] = recombine(a[0], a[2], a[1], a[3]);
+  }
+#pragma unroll
+  for (int e = 0; e < CNT; e++) {
+    int y = b[e];
+    if (e > 0) y = (int)(lift(y) - lift(w[K0 + e - 1]));  // - w_{k-1}
+#pragma unroll
+    for (int q = 2; q <= e; q += 2) {
+      // minus (the negated coefficient) products of w_{k-1-i}, i = q-1 and q
+      const int t = q + 1 <= e ? smul2(w[K0 + e - q], (int)kCoefs.cm[q - 1], w[K0 + e - q - 1], (int)kCoefs.cm[q])
+                               : smul(w[K0 + e - q], (int)kCoefs.cm[q - 1]);
+      y = (int)(lift(y) - lift(t));
+    }
+    w[K0 + e] = sbox(y);
+  }
+}
+
+// The rounds of one permutation after its first layer's products: leaves the last
+// S-box outputs in the Z columns (their layer belongs to the next product).
+__device__ __forceinline__ void rounds(Group &g) {
+#pragma unroll 1
+  for (int r = 0; r < 4; r++) {
+    if (r == 0)
+      full_sbox<false>(g);
+    else
+      full_sbox<true>(g);
+    arrive(g);
+    if (g.lead) {
+      const int off = r < 3 ? I_EXT : I_Y;
+      mma_slab(g, COL_D, COL_Z, off, 64, false);
+      mma_slab(g, COL_D, COL_Z + 8, off + SLAB64, 64, true);
+      mma_slab(g, COL_D, COL_W + 8, S_C + (r + 1) * SLAB64, 64, true);
+    }
+    finish(g);
+  }
+  {
+    int w[13];
+    uint32_t o[5];
+    partial_block<0, 4>(g, w);
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[e] = (uint32_t)w[e] + P;
+    st4(g.tw + COL_W, o);
+    arrive(g);
+    if (g.lead) mma_slab(g, COL_D + 16, COL_W, I_B2, 48, true);
+    finish(g);
+    partial_block<4, 4>(g, w);
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[e] = (uint32_t)w[4 + e] + P;
+    st4(g.tw + COL_W + 4, o);
+    arrive(g);
+    if (g.lead) mma_slab(g, COL_D + 32, COL_W, I_B3, 32, true);
+    finish(g);
+    partial_block<8, 5>(g, w);
+#pragma unroll
+    for (int e = 0; e < 5; e++) o[e] = (uint32_t)w[8 + e] + P;
+    st4(g.tw + COL_W + 8, o);
+    st1(g.tw + COL_W + 12, o[4]);
+    arrive(g);
+    if (g.lead) {
+      mma_slab(g, COL_D, COL_Z, I_O, 64, false);
+      mma_slab(g, COL_D, COL_Z + 8, I_O + SLAB64, 64, true);
+      mma_slab(g, COL_D, COL_W, I_O + 2 * SLAB64, 64, true);
+      mma_slab(g, COL_D, COL_W + 8, I_O + 3 * SLAB64, 64, true);
+    }
+    finish(g);
+  }
+#pragma unroll 1
+  for (int r = 0; r < 4; r++) {
+    if (r == 0)
+      full_sbox<false>(g);
+    else
+      full_sbox<true>(g);
+    if (r == 3) break;
+    arrive(g);
+    if (g.lead) {
+      mma_slab(g, COL_D, COL_Z, I_EXT, 64, false);
+      mma_slab(g, COL_D, COL_Z + 8, I_EXT + SLAB64, 64, true);
+      mma_slab(g, COL_D, COL_W + 8, S_C + (r + 5) * SLAB64, 64, true);
+    }
+    finish(g);
+  }
+}
+
+// The last S-box outputs, as `rounds` left them.
+__device__ __forceinline__ void load_z(const Group &g, uint32_t (&z)[16]) {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  ld16(z, g.tw + COL_Z);
+  ld_wait(z);
+}
+
+// First layer of an absorb step whose (canonical) input words are in x: `fresh` when the
+// state before it is zero, `off` the absorb matrices (S_IN or S_LAST).
+__device__ __forceinline__ void absorb(Group &g, const uint32_t (&x)[8], bool fresh, int off) {
+  st8(g.tw + COL_W, x);
+  arrive(g);
+  if (g.lead) {
+    mma_slab(g, COL_D, COL_W, off + 2 * SLAB64, 64, false);
+    mma_slab(g, COL_D, COL_W + 8, S_C, 64, true);
+    if (!fresh) {
+      mma_slab(g, COL_D, COL_Z, off, 64, true);
+      mma_slab(g, COL_D, COL_Z + 8, off + SLAB64, 64, true);
+    }
+  }
+  finish(g);
+}
+// First layer of a permutation of 16 canonical words.
+__device__ __forceinline__ void enter16(Group &g, const uint32_t (&x)[16]) {
+  st8(g.tw + COL_Z, x);
+  st8(g.tw + COL_Z + 8, x + 8);
+  arrive(g);
+  if (g.lead) {
+    mma_slab(g, COL_D, COL_Z, S_IN, 64, false);
+    mma_slab(g, COL_D, COL_Z + 8, S_IN + SLAB64, 64, true);
+    mma_slab(g, COL_D, COL_W + 8, S_C, 64, true);
+  }
+  finish(g);
+}
+// The last layer: the first OUT state words, canonical.
+template <int OUT>
+__device__ __forceinline__ void leave(Group &g, uint32_t (&o)[OUT]) {
+  arrive(g);
+  if (g.lead) {
+    mma_slab(g, COL_D, COL_Z, S_FIN, 4 * OUT, false);
+    mma_slab(g, COL_D, COL_Z + 8, S_FIN + 32 * 4 * OUT, 4 * OUT, true);
+  }
+  finish(g);
+#pragma unroll
+  for (int q = 0; q < OUT / 4; q++) {
+    uint32_t a[16];
+    ld16(a, g.tw + COL_D + 16 * q);
+    ld_wait(a);
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      o[4 * q + e] = BabyBear::red(lift(recombine(a[4 * e], a[4 * e + 2], a[4 * e + 1], a[4 * e + 3])));
+  }
+}
+
+// TMEM columns of a block of `groups` groups (a power of two).
+__host__ __device__ constexpr uint32_t tmem_cols(int groups) { return groups == 1 ? 128 : groups == 2 ? 256 : 512; }
+
+// Block set-up: tables, TMEM, barriers.  Every thread calls it; blockDim = groups * GROUP.
+__device__ __forceinline__ Group setup(uint8_t *sm, const P2Params<BabyBear, 16> &p, Mode mode, int last_rem,
+                                       uint32_t *err) {
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm), ctrl = base + smem_tables(mode);
+  const uint32_t tables = ctrl + 8;  // mbarrier of the image copies
+  const int groups = blockDim.x / GROUP;
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tables) : "memory");
+    for (int i = 0; i < groups; i++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ctrl + 16 + 8 * i) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    copy_image(base, mode, last_rem, tables);
+  }
+  for (int t = threadIdx.x; t < 8 * SLAB64 / 16; t += blockDim.x)
+    reinterpret_cast<uint4 *>(sm + S_C)[t] = make_uint4(0, 0, 0, 0);
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ctrl),
+                 "r"(tmem_cols(groups))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  if (!wait_parity(tables, 0, WAIT_POLLS)) atomicAdd(err, 1u);
+  put_constants(sm, p);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // warp-uniform by construction; the shuffles let the compiler keep them in uniform registers
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x / 32, 0), gi = warp / 4;
+  Group g;
+  g.sm = base;
+  g.tm = __shfl_sync(0xFFFFFFFFu, *reinterpret_cast<volatile uint32_t *>(sm + smem_tables(mode)), 0) + gi * COLS;
+  g.tw = g.tm + ((warp % 4) << 21);
+  g.mbar = ctrl + 16 + 8 * gi;
+  g.phase = 0;
+  g.bar = 1 + gi;
+  g.lead = warp % 4 == 0;
+  g.one = threadIdx.x % GROUP == 0;
+  g.polls = WAIT_POLLS;
+  g.err = err;
+  st1(g.tw + COL_W + W_ONE, 1);
+  return g;
+}
+__device__ __forceinline__ void teardown(uint8_t *sm, Mode mode) {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(
+                     *reinterpret_cast<volatile uint32_t *>(sm + smem_tables(mode))),
+                 "r"(tmem_cols(blockDim.x / GROUP))
+                 : "memory");
+  }
+}
+#endif  // __CUDACC__
+
+}  // namespace p2t
+}  // namespace zkb

@@ -1,6 +1,7 @@
 // poseidon2.cu — batch Poseidon2 permutation (Poseidon2Accelerator::batch_permute_*).
 #include "common.cuh"
 #include "engine.cuh"
+#include "p2_launch.cuh"
 #include "poseidon2.cuh"
 
 namespace zkb {
@@ -60,6 +61,9 @@ template <class F, int W>
 int p2_permute_batch(typename F::T *d_states, size_t n_states, const P2Params<F, W> &p,
                      cudaStream_t s) {
   if (n_states == 0) return ZKB_OK;
+  if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
+    if (p2t::takes(p, n_states)) return p2t::permute(d_states, n_states, p, s);
+  }
   DeviceContext *ctx;
   ZKB_TRY(current_context(&ctx));
   const unsigned threads = 128;
