@@ -65,6 +65,20 @@ struct BabyBear {
     uint32_t m = (uint32_t)t * NPINV;
     return red((uint32_t)((t + (uint64_t)m * P) >> 32));
   }
+#ifdef __CUDACC__
+  // Signed Montgomery product: any int32 operands (the result, hi(a b) - hi(m p), lies in
+  // (-2^31, 2^31), and in (-p, p) for |a b| < 2^31 p).  Three multiplies and a subtraction.
+  __device__ __forceinline__ static int smul(int a, int b) {
+    const int64_t t = (int64_t)a * b;
+    const int m = (int)((uint32_t)t * PINV);
+    return (int)(t >> 32) - __mulhi(m, (int)P);
+  }
+#endif
+  // [-p, p) -> [0, p); also [-p, 1.06 p] -> [0, 1.06 p]
+  __host__ __device__ __forceinline__ static uint32_t lift(int x) {
+    const uint32_t a = (uint32_t)x, b = a + P;
+    return a < b ? a : b;
+  }
   // Fully reduced Montgomery product (both operands < p).
   __host__ __device__ __forceinline__ static uint32_t mont(uint32_t a, uint32_t b) {
     return red(mont_lazy(a, b));

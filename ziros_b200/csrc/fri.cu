@@ -16,6 +16,7 @@
 #include "field.cuh"
 #include "fri_fold.cuh"
 #include "p2_launch.cuh"
+#include "p2_quad.cuh"
 
 namespace zkb {
 
@@ -97,8 +98,8 @@ __global__ void fri_fold_ext4_kernel(const uint32_t *__restrict__ e, uint32_t *_
 
 // The next FRI layer's leaves while it is made.  Leaf j of a layer is the sponge digest
 // of its codeword's rows 2j and 2j+1 flattened to 8 base elements (one permutation);
-// with FOLD each thread first folds its four input rows 4j..4j+3 (the two pairs that
-// become rows 2j and 2j+1) and stores them, so the new codeword is hashed from
+// with FOLD each quad first folds its four input rows 4j..4j+3 (the two pairs that
+// become rows 2j and 2j+1, one to each of the first two lanes of a quad) and stores them, so the new codeword is hashed from
 // registers instead of being read back.  Without FOLD it hashes the codeword `e` itself
 // (round 0).  n_leaves = 2^(log_out - 1), the output codeword holding 2^log_out rows.
 template <bool FOLD>
@@ -106,26 +107,27 @@ __global__ void __launch_bounds__(128)
     fri_fold_hash_kernel(const uint32_t *__restrict__ e, uint32_t *__restrict__ out, uint64_t n_leaves, int log_out,
                          const Ext4Params prm, const uint32_t *__restrict__ itw, uint32_t *__restrict__ digests,
                          const __grid_constant__ P2Params<BabyBear, 16> p) {
-  using D = Dom<BabyBear>;
-  for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_leaves;
-       j += (uint64_t)gridDim.x * blockDim.x) {
+  using B = BabyBear;
+  __shared__ quad::Consts<B> k;
+  quad::load_consts<B, 16>(k, p);
+  const quad::Lane l = quad::lane();
+  QUAD_ITEMS(l, j, live, n_leaves) {
     const uint4 *in = reinterpret_cast<const uint4 *>(e);
-    uint4 a, b;
-    if constexpr (FOLD) {
-      a = fold_ext4_one(in[4 * j], in[4 * j + 1], 2 * j, log_out, prm, itw);
-      b = fold_ext4_one(in[4 * j + 2], in[4 * j + 3], 2 * j + 1, log_out, prm, itw);
-      reinterpret_cast<uint4 *>(out)[2 * j] = a;
-      reinterpret_cast<uint4 *>(out)[2 * j + 1] = b;
-    } else {
-      a = in[2 * j];
-      b = in[2 * j + 1];
+    uint32_t s[4] = {0, 0, 0, 0};
+    if (l.q < 2) {  // one row to a lane
+      const uint64_t i = 2 * j + l.q;
+      uint4 a;
+      if constexpr (FOLD) {
+        a = fold_ext4_one(in[2 * i], in[2 * i + 1], i, log_out, prm, itw);
+        if (live) reinterpret_cast<uint4 *>(out)[i] = a;
+      } else {
+        a = in[i];
+      }
+      s[0] = a.x, s[1] = a.y, s[2] = a.z, s[3] = a.w;
+      quad::enter<B>(s);
     }
-    uint32_t st[16] = {D::enter(a.x), D::enter(a.y), D::enter(a.z), D::enter(a.w),
-                       D::enter(b.x), D::enter(b.y), D::enter(b.z), D::enter(b.w), 0, 0, 0, 0, 0, 0, 0, 0};
-    p2_permute<BabyBear, 16>(st, p);
-    uint4 *dg = reinterpret_cast<uint4 *>(digests) + 2 * j;
-    dg[0] = make_uint4(D::leave(st[0]), D::leave(st[1]), D::leave(st[2]), D::leave(st[3]));
-    dg[1] = make_uint4(D::leave(st[4]), D::leave(st[5]), D::leave(st[6]), D::leave(st[7]));
+    quad::permute<B, 16>(s, k, l.q);
+    if (live && l.q < 2) quad::store_words<B>(digests + j * 8 + 4 * l.q, s);
   }
 }
 
@@ -144,7 +146,7 @@ static int fold_params(const uint32_t beta[4], Ext4Params *prm) {
 static int fri_fold_hash_dev(const uint32_t *cw_in, uint32_t *cw_out, int log_out, const uint32_t *beta,
                              uint32_t *leaf_digests, const P2Params<BabyBear, 16> &p, cudaStream_t s) {
   const uint64_t n_leaves = 1ull << (log_out - 1);
-  const unsigned grid = grid_for(n_leaves, 128, 1u << 30);  // one leaf per thread
+  const unsigned grid = quad::grid_of(n_leaves, 128);  // one leaf per quad
   if (beta) {
     Ext4Params prm;
     ZKB_TRY(fold_params(beta, &prm));

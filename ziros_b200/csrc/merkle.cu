@@ -19,6 +19,7 @@
 #include "engine.cuh"
 #include "matlist.cuh"
 #include "p2_launch.cuh"
+#include "p2_quad.cuh"
 #include "poseidon2.cuh"
 
 namespace zkb {
@@ -62,126 +63,61 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// The leaf sponge of one BabyBear matrix with the alpha-reduction of each row fused in:
-// while the row streams through the sponge, out[row] accumulates sum_j alpha^j * row[j]
-// (four Montgomery products per element, 64-bit sums reduced once; the powers are
-// encoded alpha^j * 2^64 so one reduction gives the canonical sum).
+// The leaf sponge of one BabyBear matrix with the alpha-reduction of each row fused in, or of a slab
+// [c0, c0 + ncols) of its columns (row stride `stride`) when it arrives a slab at a time.
+// While the row streams through the sponge, comb[row] accumulates sum_j alpha^j * row[j]
+// (apow, when given: alpha^j * 2^64 encoded; two columns per reduction, v0*w0 + v1*w1 < 2p^2 <
+// p*2^32).  The sponge state comes from `carry` (16 words per row, internal domain; none on the
+// first slab) and goes back there, or on the last slab the digest goes to `digests`.  c0 is a
+// multiple of 8 (slabs hold whole absorbed chunks; only the last may end in a partial one),
+// so the chunks and permutations are exactly the full row's; the slabs' reductions add up to
+// the row's.
 __global__ void __launch_bounds__(128)
-    hash_rows_combine_kernel(const uint32_t *__restrict__ mat, uint64_t width, uint64_t height,
-                             uint32_t *__restrict__ digests, const __grid_constant__ P2Params<BabyBear, 16> p,
-                             const uint4 *__restrict__ apow, uint4 *__restrict__ comb) {
-  using D = Dom<BabyBear>;
+    quad_slab_kernel(const uint32_t *__restrict__ mat, uint64_t stride, uint64_t c0, uint64_t ncols, uint64_t height,
+                     uint32_t *__restrict__ carry, int first, int last, uint32_t *__restrict__ digests,
+                     const __grid_constant__ P2Params<BabyBear, 16> p, const uint4 *__restrict__ apow,
+                     uint4 *__restrict__ comb) {
   using B = BabyBear;
-  for (uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; row < height;
-       row += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t s[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) s[i] = 0;
-    // Two columns per reduction: v0*w0 + v1*w1 < 2p^2 < p*2^32 is one Montgomery
-    // reduction's input, so a pair costs two wide multiply-adds and one reduction.
-    uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-    const uint32_t *rp = mat + row * width;
-    for (uint64_t c = 0; c < width; c += 8) {
-#pragma unroll
-      for (int i = 0; i < 8; i += 2) {
-        if (c + i < width) {
-          const uint32_t v0 = rp[c + i];
-          const uint4 w0 = apow[c + i];
-          s[i] = D::enter(v0);
-          uint32_t v1 = 0;
-          uint4 w1 = make_uint4(0, 0, 0, 0);
-          if (c + i + 1 < width) {
-            v1 = rp[c + i + 1];
-            w1 = apow[c + i + 1];
-            s[i + 1] = D::enter(v1);
-          }
-          a0 += B::mont_lazy_sum(v0, w0.x, v1, w1.x);
-          a1 += B::mont_lazy_sum(v0, w0.y, v1, w1.y);
-          a2 += B::mont_lazy_sum(v0, w0.z, v1, w1.z);
-          a3 += B::mont_lazy_sum(v0, w0.w, v1, w1.w);
-        }
-      }
-      p2_permute<BabyBear, 16>(s, p);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) digests[row * 8 + i] = D::leave(s[i]);
-    comb[row] = make_uint4(B::mont_reduce(a0), B::mont_reduce(a1), B::mont_reduce(a2), B::mont_reduce(a3));
-  }
-}
-
-// The same sponge over columns [c0, c0 + ncols) of the rows only (row stride `stride`), for a
-// matrix that arrives a slab of columns at a time: the sponge state comes from `carry`
-// (16 words per row, internal domain; none on the first slab) and goes back there, or on
-// the last slab the digest goes to `digests`.  c0 is a multiple of 8 (slabs hold whole
-// absorbed chunks; only the last slab may end in a partial one), so the chunks and
-// permutations are exactly the full row's.  With apow, the rows' alpha-reduction over
-// these columns is written (first slab) or added (mod p) to comb: the sum of the slabs'
-// reductions is the whole row's.
-__global__ void __launch_bounds__(128)
-    hash_rows_slab_kernel(const uint32_t *__restrict__ mat, uint64_t stride, uint64_t c0, uint64_t ncols,
-                          uint64_t height, uint32_t *__restrict__ carry, int first, int last,
-                          uint32_t *__restrict__ digests, const __grid_constant__ P2Params<BabyBear, 16> p,
-                          const uint4 *__restrict__ apow, uint4 *__restrict__ comb) {
-  using D = Dom<BabyBear>;
-  using B = BabyBear;
-  for (uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; row < height;
-       row += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t s[16];
-    if (first) {
-#pragma unroll
-      for (int i = 0; i < 16; i++) s[i] = 0;
-    } else {
-      const uint4 *cp = reinterpret_cast<const uint4 *>(carry + row * 16);
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint4 v = cp[q];
-        s[4 * q] = v.x;
-        s[4 * q + 1] = v.y;
-        s[4 * q + 2] = v.z;
-        s[4 * q + 3] = v.w;
-      }
-    }
+  __shared__ quad::Consts<B> k;
+  quad::load_consts<B, 16>(k, p);
+  const quad::Lane l = quad::lane();
+  QUAD_ITEMS(l, row, live, height) {
+    uint32_t s[4] = {0, 0, 0, 0};
+    if (!first) quad::load_words<uint32_t>(s, carry + row * 16 + 4 * l.q);
     uint64_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
     const uint32_t *rp = mat + row * stride + c0;
     const uint4 *ap = apow ? apow + c0 : nullptr;
-    for (uint64_t c = 0; c < ncols; c += 8) {
+    quad::absorb<B, 16, true>(
+        s, ncols, k, l.q, [&](uint64_t c) { return rp[c]; },
+        [&](const uint32_t(&x)[4], uint64_t c) {
+          if (!ap) return;
 #pragma unroll
-      for (int i = 0; i < 8; i += 2) {
-        if (c + i < ncols) {
-          const uint32_t v0 = rp[c + i];
-          s[i] = D::enter(v0);
-          uint32_t v1 = 0;
-          if (c + i + 1 < ncols) {
-            v1 = rp[c + i + 1];
-            s[i + 1] = D::enter(v1);
-          }
-          if (ap) {
+          for (int i = 0; i < 4; i += 2) {
+            if (c + i >= ncols) break;
             const uint4 w0 = ap[c + i];
             const uint4 w1 = c + i + 1 < ncols ? ap[c + i + 1] : make_uint4(0, 0, 0, 0);
-            a0 += B::mont_lazy_sum(v0, w0.x, v1, w1.x);
-            a1 += B::mont_lazy_sum(v0, w0.y, v1, w1.y);
-            a2 += B::mont_lazy_sum(v0, w0.z, v1, w1.z);
-            a3 += B::mont_lazy_sum(v0, w0.w, v1, w1.w);
+            a0 += B::mont_lazy_sum(x[i], w0.x, x[i + 1], w1.x);
+            a1 += B::mont_lazy_sum(x[i], w0.y, x[i + 1], w1.y);
+            a2 += B::mont_lazy_sum(x[i], w0.z, x[i + 1], w1.z);
+            a3 += B::mont_lazy_sum(x[i], w0.w, x[i + 1], w1.w);
           }
+        });
+    if (!last) {
+      if (live) *reinterpret_cast<uint4 *>(carry + row * 16 + 4 * l.q) = make_uint4(s[0], s[1], s[2], s[3]);
+    } else if (live && l.q < 2) {
+      quad::store_words<B>(digests + row * 8 + 4 * l.q, s);
+    }
+    if (ap) {  // the first two lanes have the sums of their columns
+      uint32_t r[4] = {B::mont_reduce(a0), B::mont_reduce(a1), B::mont_reduce(a2), B::mont_reduce(a3)};
+#pragma unroll
+      for (int i = 0; i < 4; i++) r[i] = B::add(r[i], __shfl_xor_sync(0xFFFFFFFFu, r[i], 1));
+      if (live && l.q == 0) {
+        if (!first) {
+          const uint4 o = comb[row];
+          r[0] = B::add(o.x, r[0]), r[1] = B::add(o.y, r[1]), r[2] = B::add(o.z, r[2]), r[3] = B::add(o.w, r[3]);
         }
+        comb[row] = make_uint4(r[0], r[1], r[2], r[3]);
       }
-      p2_permute<BabyBear, 16>(s, p);
-    }
-    if (last) {
-#pragma unroll
-      for (int i = 0; i < 8; i++) digests[row * 8 + i] = D::leave(s[i]);
-    } else {
-      uint4 *cp = reinterpret_cast<uint4 *>(carry + row * 16);
-#pragma unroll
-      for (int q = 0; q < 4; q++) cp[q] = make_uint4(s[4 * q], s[4 * q + 1], s[4 * q + 2], s[4 * q + 3]);
-    }
-    if (ap) {
-      uint4 r = make_uint4(B::mont_reduce(a0), B::mont_reduce(a1), B::mont_reduce(a2), B::mont_reduce(a3));
-      if (!first) {
-        const uint4 o = comb[row];
-        r = make_uint4(B::add(o.x, r.x), B::add(o.y, r.y), B::add(o.z, r.z), B::add(o.w, r.w));
-      }
-      comb[row] = r;
     }
   }
 }
@@ -317,33 +253,48 @@ static int build_tree_impl(const HasherSpec &h, const std::vector<TreeMatrix> &m
   // jobs higher stream priority) get SMs in between instead of waiting for the whole grid.
   const unsigned cap = 1u << 30;
   (void)ctx;
+  // Leaf digests of the matrices in `l` (rows of one height).
+  auto hash = [&](const MatList &l, uint64_t height, T *out, const LeafCombine *c, const char *name) -> int {
+    if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
+      if (l.col_start[l.n] > 0 && p2t::takes(p, height))
+        return p2t::hash_rows(l, height, out, p, c ? c->apow : nullptr, c ? c->out : nullptr, name, s);
+      if (c) {
+        ZKB_LAUNCH(name, s, quad_slab_kernel<<<quad::grid_of(height, thr), thr, 0, s>>>((const uint32_t *)l.ptr[0], l.width[0], 0, l.width[0], height, nullptr, 1, 1, out, p, c->apow, c->out));
+        return ZKB_OK;
+      }
+    }
+    if (quad::takes<F, W>(height)) {
+      ZKB_LAUNCH(name, s, quad::rows_kernel<F, W><<<quad::grid_of(height, thr), thr, 0, s>>>(l, height, out, p));
+    } else if constexpr (!std::is_same<F, BabyBear>::value) {
+      ZKB_LAUNCH(name, s, hash_rows_kernel<F, W><<<grid_for(height, thr, cap), thr, 0, s>>>(l, height, out, p));
+    }
+    return ZKB_OK;
+  };
   if (fill) {
     // the caller writes layer 0 (e.g. slab by slab as the matrix arrives)
     ZKB_REQUIRE(nm == 1 && comb == nullptr, "internal: leaves written by the caller take one matrix");
     ZKB_TRY((*fill)(layers));
-  } else if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
-    if (comb) ZKB_REQUIRE(nm == 1, "the fused alpha-reduction takes one matrix");
-    if (ml.col_start[ml.n] > 0 && p2t::takes(p, max_h)) {
-      ZKB_TRY(p2t::hash_rows(ml, max_h, layers, p, comb ? comb->apow : nullptr, comb ? comb->out : nullptr, leaf_name, s));
-    } else if (comb) {
-      ZKB_LAUNCH(leaf_name, s, hash_rows_combine_kernel<<<grid_for(max_h, thr, cap), thr, 0, s>>>((const uint32_t *)ml.ptr[0], ml.width[0], max_h, layers, p, comb->apow, comb->out));
-    } else {
-      ZKB_LAUNCH(leaf_name, s, hash_rows_kernel<F, W><<<grid_for(max_h, thr, cap), thr, 0, s>>>(ml, max_h, layers, p));
-    }
   } else {
-    ZKB_REQUIRE(comb == nullptr, "the fused alpha-reduction is BabyBear width 16 only");
-    ZKB_LAUNCH(leaf_name, s, hash_rows_kernel<F, W><<<grid_for(max_h, thr, cap), thr, 0, s>>>(ml, max_h, layers, p));
+    if (comb) {
+      ZKB_REQUIRE(h.field == FIELD_BABYBEAR, "the fused alpha-reduction is BabyBear width 16 only");
+      ZKB_REQUIRE(nm == 1, "the fused alpha-reduction takes one matrix");
+    }
+    ZKB_TRY(hash(ml, max_h, layers, comb, leaf_name));
   }
-  ZKB_CHECK_LAUNCH();
   ScratchBuf inj_buf;  // digests of rows injected at one layer (sized for the largest)
 
   size_t next_m = ng;
-  for (size_t li = 0; li + 1 < t->layer_len.size(); li++) {
-    const uint64_t prev_len = t->layer_len[li];
-    const uint64_t half = prev_len / 2;
-    const uint64_t next_layer_len = next_pow2_u64(half);
+  // the matrices injected when layer li is compressed
+  auto injected = [&](size_t li) {
+    const uint64_t next_layer_len = next_pow2_u64(t->layer_len[li] / 2);
     size_t ni = 0;
     while (next_m + ni < nm && next_pow2_u64(mats[ord[next_m + ni]].height) == next_layer_len) ni++;
+    return ni;
+  };
+  const size_t top = t->layer_len.size() - 1;
+  for (size_t li = 0; li < top; li++) {
+    const uint64_t half = t->layer_len[li] / 2;
+    const size_t ni = injected(li);
     const T *prev = layers + t->layer_off[li] * OUT;
     T *next = layers + t->layer_off[li + 1] * OUT;
     const T *inj = nullptr;
@@ -353,13 +304,7 @@ static int build_tree_impl(const HasherSpec &h, const std::vector<TreeMatrix> &m
       ZKB_TRY(make_list(next_m, ni, &iml));
       inj_h = mats[ord[next_m]].height;
       if (!inj_buf.p) ZKB_TRY(inj_buf.alloc(inj_h * OUT * sizeof(T), s));
-      bool tensor = false;
-      if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
-        tensor = iml.col_start[iml.n] > 0 && p2t::takes(p, inj_h);
-        if (tensor) ZKB_TRY(p2t::hash_rows(iml, inj_h, inj_buf.as<T>(), p, nullptr, nullptr, "merkle_inject_hash", s));
-      }
-      if (!tensor)
-        ZKB_LAUNCH("merkle_inject_hash", s, hash_rows_kernel<F, W><<<grid_for(inj_h, thr, cap), thr, 0, s>>>(iml, inj_h, inj_buf.as<T>(), p));
+      ZKB_TRY(hash(iml, inj_h, inj_buf.as<T>(), nullptr, "merkle_inject_hash"));
       inj = inj_buf.as<T>();
     }
     next_m += ni;
@@ -369,7 +314,30 @@ static int build_tree_impl(const HasherSpec &h, const std::vector<TreeMatrix> &m
         continue;
       }
     }
-    ZKB_LAUNCH(comp_name, s, compress_kernel<F, W><<<grid_for(half, thr, cap), thr, 0, s>>>(prev, next, half, inj, inj_h, p));
+    if (quad::takes<F, W>(half)) {
+      if (inj) {
+        ZKB_LAUNCH(comp_name, s, quad::inject_kernel<F, W><<<quad::grid_of(half, thr), thr, 0, s>>>(prev, next, half, inj, inj_h, p));
+        continue;
+      }
+      // every level up to the next injection, a few launches of whole subtrees
+      size_t end = li + 1;
+      while (end < top && injected(end) == 0) end++;
+      const int levels = quad::run_levels((int)(end - li));
+      for (size_t at = li; at < end; at += levels) {
+        const int n = (int)std::min<size_t>(levels, end - at);
+        quad::Run run{};
+        run.layers = layers;
+        for (int j = 0; j <= n; j++) {
+          run.off[j] = t->layer_off[at + j];
+          run.n[j] = j || at > 0 ? t->layer_len[at + j - 1] / 2 : max_h;
+        }
+        const uint64_t nodes = t->layer_len[at];
+        ZKB_LAUNCH(comp_name, s, quad::levels_kernel<F, W><<<(unsigned)((nodes + (1ull << n) - 1) >> n), quad::run_threads(n), quad::run_smem<F, W>(n), s>>>(run, n, p));
+      }
+      li = end - 1;
+    } else if constexpr (!std::is_same<F, BabyBear>::value) {
+      ZKB_LAUNCH(comp_name, s, compress_kernel<F, W><<<grid_for(half, thr, cap), thr, 0, s>>>(prev, next, half, inj, inj_h, p));
+    }
   }
   return ZKB_OK;
 }
@@ -399,7 +367,7 @@ int hash_rows_slab_dev(const HasherSpec &h, const uint32_t *mat, uint64_t stride
   if (p2t::takes(p, height))  // by the height alone: every slab of a matrix takes the same form
     return p2t::hash_slab(mat, stride, c0, ncols, height, carry, first, last, digests, p, apow, out, "merkle_leaf_hash", s);
   const unsigned thr = 128;
-  ZKB_LAUNCH("merkle_leaf_hash", s, hash_rows_slab_kernel<<<grid_for(height, thr, 1u << 30), thr, 0, s>>>(mat, stride, c0, ncols, height, carry, first ? 1 : 0, last ? 1 : 0, digests, p, apow, out));
+  ZKB_LAUNCH("merkle_leaf_hash", s, quad_slab_kernel<<<quad::grid_of(height, thr), thr, 0, s>>>(mat, stride, c0, ncols, height, carry, first ? 1 : 0, last ? 1 : 0, digests, p, apow, out));
   return ZKB_OK;
 }
 

@@ -12,6 +12,7 @@
 
 #include "common.cuh"
 #include "p2_launch.cuh"
+#include "p2_quad.cuh"
 #include "poseidon2.cuh"
 
 namespace zkb {
@@ -232,16 +233,36 @@ int launch_trees(const Tables &t, const LeafJob *d_leaf, const CompJob *d_comp, 
       leaves_done = true;
     }
   }
-  if (!leaves_done)
-    ZKB_LAUNCH(leaf_name, s, mt_leaf_kernel<F, W><<<grid_for(t.total_rows, leaf_threads, 1u << 30), leaf_threads, n * sizeof(uint64_t), s>>>(d_leaf, n, t.total_rows, p));
-  for (size_t l = 0; l < t.lvl_cnt.size(); l++) {
+  if (!leaves_done) {
+    if (quad::takes<F, W>(t.total_rows)) {
+      ZKB_LAUNCH(leaf_name, s, quad::mt_rows_kernel<F, W, LeafJob><<<quad::grid_of(t.total_rows, leaf_threads), leaf_threads, n * sizeof(uint64_t), s>>>(d_leaf, n, t.total_rows, p));
+    } else if constexpr (!bb16) {
+      ZKB_LAUNCH(leaf_name, s, mt_leaf_kernel<F, W><<<grid_for(t.total_rows, leaf_threads, 1u << 30), leaf_threads, n * sizeof(uint64_t), s>>>(d_leaf, n, t.total_rows, p));
+    }
+  }
+  const size_t levels = t.lvl_cnt.size();
+  size_t l = 0;
+  for (; l < levels; l++) {
     if constexpr (bb16) {
       if (p2t::takes(p, t.lvl_total[l])) {
         ZKB_TRY(p2t::mt_compress(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p, comp_name, s));
         continue;
       }
     }
-    ZKB_LAUNCH(comp_name, s, mt_compress_kernel<F, W><<<grid_for(t.lvl_total[l], 128, 1u << 30), 128, t.lvl_cnt[l] * sizeof(uint64_t), s>>>(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p));
+    if (quad::takes<F, W>(t.lvl_total[l])) break;
+    if constexpr (!bb16)
+      ZKB_LAUNCH(comp_name, s, mt_compress_kernel<F, W><<<grid_for(t.lvl_total[l], 128, 1u << 30), 128, t.lvl_cnt[l] * sizeof(uint64_t), s>>>(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p));
+  }
+  // the levels left are small ones (the totals halve from level to level): whole subtrees
+  if (l < levels) {
+    const int step = quad::run_levels((int)(levels - l));
+    for (; l < levels; l += step) {
+      const int run = (int)std::min<size_t>(step, levels - l);
+      uint64_t blocks = 0;
+      for (const LeafJob &j : t.leaf)
+        if (const uint64_t nodes = j.rows >> l; nodes >= 2) blocks += (nodes + (1ull << run) - 1) >> run;
+      ZKB_LAUNCH(comp_name, s, quad::mt_levels_kernel<F, W, LeafJob><<<(unsigned)blocks, quad::run_threads(run), quad::run_smem<F, W>(run), s>>>(d_leaf, n, (int)l, run, p));
+    }
   }
   ZKB_LAUNCH(root_name, s, mt_roots_kernel<T, OUT><<<(n * OUT + 127) / 128, 128, 0, s>>>(d_root_off, (const T *)base, n, d_root_dst, (T *)d_roots));
   return ZKB_OK;

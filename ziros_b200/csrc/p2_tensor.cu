@@ -376,8 +376,10 @@ static int prepare(K kernel, size_t smem) {
   return ZKB_OK;
 }
 
-// Smallest number of rows (or compressions) in one launch.
-constexpr uint64_t MIN_ROWS = 148ull * GROUP * 5 / 2;
+// Smallest number of rows (or compressions) in one launch: more than one tile an SM.  Up to there
+// the quad form is the faster one (16,384 rows x 32 columns: 46 us against 55; 18,944 x 64: 86
+// against 91), from there this one (32,768 x 8: 21.5 us against 24.7, x 64: 109 against 135).
+constexpr uint64_t MIN_ROWS = 148ull * GROUP + 1;
 
 bool takes(const P2Params<BabyBear, 16> &p, uint64_t rows) { return usable(p) && rows >= MIN_ROWS; }
 

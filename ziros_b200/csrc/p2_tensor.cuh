@@ -328,14 +328,8 @@ __device__ __forceinline__ void ld_wait(uint32_t (&v)[16]) {
 }
 
 // --------------------------------------------------------------------- arithmetic
-// Signed Montgomery product: any int32 operands (the result, hi(a b) - hi(m p), lies in
-// (-2^31, 2^31), and in (-p, p) for |a b| < 2^31 p).  Five multiplier issue slots: a wide
-// product, a low one, a high one.
-__device__ __forceinline__ int smul(int a, int b) {
-  const int64_t t = (int64_t)a * b;
-  const int m = (int)((uint32_t)t * BabyBear::PINV);
-  return (int)(t >> 32) - __mulhi(m, (int)P);
-}
+__device__ __forceinline__ int smul(int a, int b) { return BabyBear::smul(a, b); }
+__device__ __forceinline__ uint32_t lift(int x) { return BabyBear::lift(x); }
 __device__ __forceinline__ int smul2(int a0, int b0, int a1, int b1) {
   const int64_t t = (int64_t)a0 * b0 + (int64_t)a1 * b1;
   const int m = (int)((uint32_t)t * BabyBear::PINV);
@@ -348,11 +342,6 @@ __device__ __forceinline__ int sbox(int x) {
   const int x3 = smul(x2, x);
   const int x4 = smul(x2, x2);
   return smul(x3, x4);
-}
-// [-p, p) -> [0, p); also [-p, 1.06 p] -> [0, 1.06 p]
-__device__ __forceinline__ uint32_t lift(int x) {
-  const uint32_t a = (uint32_t)x, b = a + P;
-  return a < b ? a : b;
 }
 // The output word of four accumulators, congruent to a0 + a1 2^8 + a2 2^16 + a3 2^24 mod p and in
 // [-p, 1.04 p]: u = a0 + a1 2^8 and v = a2 + a3 2^8 stay below 0.97 p (at most 120 operand

@@ -2,6 +2,7 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "p2_launch.cuh"
+#include "p2_quad.cuh"
 #include "poseidon2.cuh"
 
 namespace zkb {
@@ -67,8 +68,12 @@ int p2_permute_batch(typename F::T *d_states, size_t n_states, const P2Params<F,
   DeviceContext *ctx;
   ZKB_TRY(current_context(&ctx));
   const unsigned threads = 128;
-  unsigned grid = grid_for(n_states, threads, (unsigned)ctx->sm_count * 16u);
-  ZKB_LAUNCH("p2_permute", s, p2_batch_kernel<F, W><<<grid, threads, 0, s>>>(d_states, n_states, p));
+  if (quad::takes<F, W>(n_states)) {
+    ZKB_LAUNCH("p2_permute", s, quad::states_kernel<F, W><<<quad::grid_of(n_states, threads), threads, 0, s>>>(d_states, n_states, p));
+  } else if constexpr (!std::is_same<F, BabyBear>::value) {
+    const unsigned grid = grid_for(n_states, threads, (unsigned)ctx->sm_count * 16u);
+    ZKB_LAUNCH("p2_permute", s, p2_batch_kernel<F, W><<<grid, threads, 0, s>>>(d_states, n_states, p));
+  }
   ZKB_CHECK_LAUNCH();
   return ZKB_OK;
 }
