@@ -281,12 +281,14 @@ int zkb_engine_submit(zkb_engine *e, const zkb_job_desc *desc, uint64_t *job_id)
                 "job needs ~%llu bytes of device memory, more than the engine budget %llu",
                 (unsigned long long)job->mem_estimate, (unsigned long long)e->budget);
     job->id = e->next_id++;
-    job->t_submit = Clock::now();
     (void)log_epoch();  // the job log's clock starts at the first submission
     e->jobs[job->id] = job;
     e->queue.push_back(job);
+    // Woken workers wait for the lock, so the time is taken before any of them sees the job, and
+    // waking them (system calls) does not lie between it and the return to the caller.
+    e->cv_queue.notify_all();
+    job->t_submit = Clock::now();
   }
-  e->cv_queue.notify_all();
   *job_id = job->id;
   return ZKB_OK;
 }
