@@ -275,10 +275,11 @@ int zkb_set_ntt_tile_loads(int mode) {
 int zkb_ntt_tile_load_errors(uint32_t *count) {
   ZKB_ENTRY();
   ZKB_REQUIRE(count != nullptr, "null count");
-  uint32_t hashing = 0;
-  ZKB_TRY(p2t::wait_errors(&hashing));
+  uint32_t bb = 0, gl = 0;
+  ZKB_TRY(p2t::wait_errors(&bb));
+  ZKB_TRY(p2g::wait_errors(&gl));
   ZKB_TRY(ntt_tma_wait_errors(count));
-  *count += hashing;
+  *count += bb + gl;
   return ZKB_OK;
 }
 

@@ -29,40 +29,6 @@ __host__ __device__ constexpr int p2_out() {
   return W == 16 ? 8 : 4;
 }
 
-// Leaf digests: PaddingFreeSponge over the concatenated row of the matrices in ml.
-// One permutation call site per kernel (keeps the code within the instruction cache);
-// a partial last chunk overwrites only its own lanes.
-template <class F, int W>
-__global__ void __launch_bounds__(128)
-    hash_rows_kernel(const MatList ml, uint64_t height, typename F::T *__restrict__ digests,
-                     const __grid_constant__ P2Params<F, W> p) {
-  using T = typename F::T;
-  using D = Dom<F>;
-  constexpr int OUT = p2_out<W>();
-  const uint64_t total = ml.col_start[ml.n];
-  for (uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; row < height;
-       row += (uint64_t)gridDim.x * blockDim.x) {
-    T s[W];
-#pragma unroll
-    for (int i = 0; i < W; i++) s[i] = 0;
-    const T *rp = (const T *)ml.ptr[0] + row * ml.width[0];
-    for (uint64_t c = 0; c < total; c += 8) {
-      if (ml.n == 1) {
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-          if (c + i < total) s[i] = D::enter(rp[c + i]);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-          if (c + i < total) s[i] = D::enter(fetch_col<F>(ml, row, c + i));
-      }
-      p2_permute<F, W>(s, p);
-    }
-#pragma unroll
-    for (int i = 0; i < OUT; i++) digests[row * OUT + i] = D::leave(s[i]);
-  }
-}
-
 // The leaf sponge of one BabyBear matrix with the alpha-reduction of each row fused in, or of a slab
 // [c0, c0 + ncols) of its columns (row stride `stride`) when it arrives a slab at a time.
 // While the row streams through the sponge, comb[row] accumulates sum_j alpha^j * row[j]
@@ -119,39 +85,6 @@ __global__ void __launch_bounds__(128)
         comb[row] = make_uint4(r[0], r[1], r[2], r[3]);
       }
     }
-  }
-}
-
-// next[i] = compress(prev[2i], prev[2i+1]); with `inj` (digests of the rows injected at
-// this layer, inj_h of them) next[i] = compress(that, i < inj_h ? inj[i] : 0).
-template <class F, int W>
-__global__ void __launch_bounds__(128)
-    compress_kernel(const typename F::T *__restrict__ prev, typename F::T *__restrict__ next,
-                    uint64_t n_out, const typename F::T *__restrict__ inj, uint64_t inj_h,
-                    const __grid_constant__ P2Params<F, W> p) {
-  using T = typename F::T;
-  using D = Dom<F>;
-  constexpr int OUT = p2_out<W>();
-  const int rounds = inj ? 2 : 1;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_out;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    T s[W];
-#pragma unroll
-    for (int k = 0; k < OUT; k++) {
-      s[k] = D::enter(prev[(2 * i) * OUT + k]);
-      s[OUT + k] = D::enter(prev[(2 * i + 1) * OUT + k]);
-    }
-    for (int r = 0; r < rounds; r++) {
-      if (r == 1) {
-#pragma unroll
-        for (int k = 0; k < OUT; k++) s[OUT + k] = i < inj_h ? D::enter(inj[i * OUT + k]) : (T)0;
-      }
-#pragma unroll
-      for (int k = 2 * OUT; k < W; k++) s[k] = 0;
-      p2_permute<F, W>(s, p);
-    }
-#pragma unroll
-    for (int k = 0; k < OUT; k++) next[i * OUT + k] = D::leave(s[k]);
   }
 }
 
@@ -251,23 +184,23 @@ static int build_tree_impl(const HasherSpec &h, const std::vector<TreeMatrix> &m
   // One row (or pair) per thread and as many blocks as that takes: blocks retire every few
   // milliseconds, so kernels of other streams (other jobs of the engine, which gives small
   // jobs higher stream priority) get SMs in between instead of waiting for the whole grid.
-  const unsigned cap = 1u << 30;
   (void)ctx;
   // Leaf digests of the matrices in `l` (rows of one height).
+  constexpr bool bb = std::is_same<F, BabyBear>::value;
   auto hash = [&](const MatList &l, uint64_t height, T *out, const LeafCombine *c, const char *name) -> int {
-    if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
-      if (l.col_start[l.n] > 0 && p2t::takes(p, height))
+    if (l.col_start[l.n] > 0 && tensor_takes<F, W>(p, height)) {
+      if constexpr (bb)
         return p2t::hash_rows(l, height, out, p, c ? c->apow : nullptr, c ? c->out : nullptr, name, s);
+      else
+        return p2g::hash_rows<W>(l, height, out, p, name, s);
+    }
+    if constexpr (bb) {
       if (c) {
         ZKB_LAUNCH(name, s, quad_slab_kernel<<<quad::grid_of(height, thr), thr, 0, s>>>((const uint32_t *)l.ptr[0], l.width[0], 0, l.width[0], height, nullptr, 1, 1, out, p, c->apow, c->out));
         return ZKB_OK;
       }
     }
-    if (quad::takes<F, W>(height)) {
-      ZKB_LAUNCH(name, s, quad::rows_kernel<F, W><<<quad::grid_of(height, thr), thr, 0, s>>>(l, height, out, p));
-    } else if constexpr (!std::is_same<F, BabyBear>::value) {
-      ZKB_LAUNCH(name, s, hash_rows_kernel<F, W><<<grid_for(height, thr, cap), thr, 0, s>>>(l, height, out, p));
-    }
+    ZKB_LAUNCH(name, s, quad::rows_kernel<F, W><<<quad::grid_of(height, thr), thr, 0, s>>>(l, height, out, p));
     return ZKB_OK;
   };
   if (fill) {
@@ -308,36 +241,33 @@ static int build_tree_impl(const HasherSpec &h, const std::vector<TreeMatrix> &m
       inj = inj_buf.as<T>();
     }
     next_m += ni;
-    if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
-      if (p2t::takes(p, half)) {
+    if (tensor_takes<F, W>(p, half)) {
+      if constexpr (bb)
         ZKB_TRY(p2t::compress(prev, next, half, inj, inj_h, p, comp_name, s));
-        continue;
-      }
+      else
+        ZKB_TRY(p2g::compress<W>(prev, next, half, inj, inj_h, p, comp_name, s));
+      continue;
     }
-    if (quad::takes<F, W>(half)) {
-      if (inj) {
-        ZKB_LAUNCH(comp_name, s, quad::inject_kernel<F, W><<<quad::grid_of(half, thr), thr, 0, s>>>(prev, next, half, inj, inj_h, p));
-        continue;
-      }
-      // every level up to the next injection, a few launches of whole subtrees
-      size_t end = li + 1;
-      while (end < top && injected(end) == 0) end++;
-      const int levels = quad::run_levels((int)(end - li));
-      for (size_t at = li; at < end; at += levels) {
-        const int n = (int)std::min<size_t>(levels, end - at);
-        quad::Run run{};
-        run.layers = layers;
-        for (int j = 0; j <= n; j++) {
-          run.off[j] = t->layer_off[at + j];
-          run.n[j] = j || at > 0 ? t->layer_len[at + j - 1] / 2 : max_h;
-        }
-        const uint64_t nodes = t->layer_len[at];
-        ZKB_LAUNCH(comp_name, s, quad::levels_kernel<F, W><<<(unsigned)((nodes + (1ull << n) - 1) >> n), quad::run_threads(n), quad::run_smem<F, W>(n), s>>>(run, n, p));
-      }
-      li = end - 1;
-    } else if constexpr (!std::is_same<F, BabyBear>::value) {
-      ZKB_LAUNCH(comp_name, s, compress_kernel<F, W><<<grid_for(half, thr, cap), thr, 0, s>>>(prev, next, half, inj, inj_h, p));
+    if (inj) {
+      ZKB_LAUNCH(comp_name, s, quad::inject_kernel<F, W><<<quad::grid_of(half, thr), thr, 0, s>>>(prev, next, half, inj, inj_h, p));
+      continue;
     }
+    // every level up to the next injection, a few launches of whole subtrees
+    size_t end = li + 1;
+    while (end < top && injected(end) == 0) end++;
+    const int levels = quad::run_levels((int)(end - li));
+    for (size_t at = li; at < end; at += levels) {
+      const int n = (int)std::min<size_t>(levels, end - at);
+      quad::Run run{};
+      run.layers = layers;
+      for (int j = 0; j <= n; j++) {
+        run.off[j] = t->layer_off[at + j];
+        run.n[j] = j || at > 0 ? t->layer_len[at + j - 1] / 2 : max_h;
+      }
+      const uint64_t nodes = t->layer_len[at];
+      ZKB_LAUNCH(comp_name, s, quad::levels_kernel<F, W><<<(unsigned)((nodes + (1ull << n) - 1) >> n), quad::run_threads(n), quad::run_smem<F, W>(n), s>>>(run, n, p));
+    }
+    li = end - 1;
   }
   return ZKB_OK;
 }

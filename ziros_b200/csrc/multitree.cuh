@@ -52,69 +52,6 @@ __device__ __forceinline__ int find_job(const uint64_t *starts, int n, uint64_t 
   return lo;
 }
 
-// PaddingFreeSponge leaf digest of every row of every job (one permutation call site).
-template <class F, int W>
-__global__ void __launch_bounds__(256)
-    mt_leaf_kernel(const LeafJob *__restrict__ jobs, int n_jobs, uint64_t total_rows,
-                   const __grid_constant__ P2Params<F, W> p) {
-  using T = typename F::T;
-  using D = Dom<F>;
-  constexpr int OUT = digest_len<W>();
-  extern __shared__ uint64_t starts[];  // n_jobs entries
-  for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].row_start;
-  __syncthreads();
-  for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total_rows;
-       g += (uint64_t)gridDim.x * blockDim.x) {
-    const int j = find_job(starts, n_jobs, g);
-    const uint64_t row = g - starts[j];
-    const uint64_t width = jobs[j].width;
-    const T *rp = (const T *)jobs[j].data + row * width;
-    T s[W];
-#pragma unroll
-    for (int i = 0; i < W; i++) s[i] = 0;
-    for (uint64_t c = 0; c < width; c += 8) {
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-        if (c + i < width) s[i] = D::enter(rp[c + i]);
-      p2_permute<F, W>(s, p);
-    }
-    T *out = (T *)jobs[j].digests + row * OUT;
-#pragma unroll
-    for (int i = 0; i < OUT; i++) out[i] = D::leave(s[i]);
-  }
-}
-
-// next[i] = compress(prev[2i], prev[2i+1]) for every job of one tree level.
-template <class F, int W>
-__global__ void __launch_bounds__(128)
-    mt_compress_kernel(const CompJob *__restrict__ jobs, int n_jobs, uint64_t total,
-                       const __grid_constant__ P2Params<F, W> p) {
-  using T = typename F::T;
-  using D = Dom<F>;
-  constexpr int OUT = digest_len<W>();
-  extern __shared__ uint64_t starts[];  // n_jobs entries
-  for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].start;
-  __syncthreads();
-  for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < total;
-       g += (uint64_t)gridDim.x * blockDim.x) {
-    const int j = find_job(starts, n_jobs, g);
-    const uint64_t i = g - starts[j];
-    const T *prev = (const T *)jobs[j].prev;
-    T s[W];
-#pragma unroll
-    for (int k = 0; k < OUT; k++) {
-      s[k] = D::enter(prev[(2 * i) * OUT + k]);
-      s[OUT + k] = D::enter(prev[(2 * i + 1) * OUT + k]);
-    }
-#pragma unroll
-    for (int k = 2 * OUT; k < W; k++) s[k] = 0;
-    p2_permute<F, W>(s, p);
-    T *next = (T *)jobs[j].next + i * OUT;
-#pragma unroll
-    for (int k = 0; k < OUT; k++) next[k] = D::leave(s[k]);
-  }
-}
-
 // roots[dst[j]] = the last digest of job j's layers (offsets in digests from `base`;
 // dst NULL: roots[j])
 template <class T, int OUT>
@@ -217,41 +154,27 @@ int launch_trees(const Tables &t, const LeafJob *d_leaf, const CompJob *d_comp, 
                  const uint32_t *d_root_dst = nullptr) {
   using T = typename F::T;
   constexpr int OUT = digest_len<W>();
-  DeviceContext *ctx;
-  ZKB_TRY(current_context(&ctx));
   const int n = (int)t.leaf.size();
-  // one row (or compression) per thread: short-lived blocks, so concurrent streams
-  // interleave at block granularity
-  (void)ctx;
-  constexpr bool bb16 = std::is_same<F, BabyBear>::value && W == 16;
-  bool leaves_done = leaf_name == nullptr;
-  if constexpr (bb16) {
+  constexpr bool bb = std::is_same<F, BabyBear>::value;
+  if (leaf_name) {
     // Tiles hold 128 rows of one job: jobs of fewer rows leave lanes idle, and with more than a
-    // quarter of the lanes idle the row-per-thread kernel is the faster one.
-    if (!leaves_done && !t.empty_rows && p2t::takes(p, t.total_rows) && t.tiles * 128 <= t.total_rows + t.total_rows / 4) {
-      ZKB_TRY(p2t::mt_leaf(d_leaf, n, t.tiles, t.max_perms, p, leaf_name, s));
-      leaves_done = true;
-    }
-  }
-  if (!leaves_done) {
-    if (quad::takes<F, W>(t.total_rows)) {
+    // quarter of the lanes idle the quads are the faster form.
+    if (!t.empty_rows && tensor_takes<F, W>(p, t.total_rows) && t.tiles * 128 <= t.total_rows + t.total_rows / 4) {
+      if constexpr (bb)
+        ZKB_TRY(p2t::mt_leaf(d_leaf, n, t.tiles, t.max_perms, p, leaf_name, s));
+      else
+        ZKB_TRY(p2g::mt_leaf<W>(d_leaf, n, t.tiles, t.max_perms, p, leaf_name, s));
+    } else {
       ZKB_LAUNCH(leaf_name, s, quad::mt_rows_kernel<F, W, LeafJob><<<quad::grid_of(t.total_rows, leaf_threads), leaf_threads, n * sizeof(uint64_t), s>>>(d_leaf, n, t.total_rows, p));
-    } else if constexpr (!bb16) {
-      ZKB_LAUNCH(leaf_name, s, mt_leaf_kernel<F, W><<<grid_for(t.total_rows, leaf_threads, 1u << 30), leaf_threads, n * sizeof(uint64_t), s>>>(d_leaf, n, t.total_rows, p));
     }
   }
   const size_t levels = t.lvl_cnt.size();
   size_t l = 0;
-  for (; l < levels; l++) {
-    if constexpr (bb16) {
-      if (p2t::takes(p, t.lvl_total[l])) {
-        ZKB_TRY(p2t::mt_compress(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p, comp_name, s));
-        continue;
-      }
-    }
-    if (quad::takes<F, W>(t.lvl_total[l])) break;
-    if constexpr (!bb16)
-      ZKB_LAUNCH(comp_name, s, mt_compress_kernel<F, W><<<grid_for(t.lvl_total[l], 128, 1u << 30), 128, t.lvl_cnt[l] * sizeof(uint64_t), s>>>(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p));
+  for (; l < levels && tensor_takes<F, W>(p, t.lvl_total[l]); l++) {
+    if constexpr (bb)
+      ZKB_TRY(p2t::mt_compress(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p, comp_name, s));
+    else
+      ZKB_TRY(p2g::mt_compress<W>(d_comp + t.lvl_off[l], (int)t.lvl_cnt[l], t.lvl_total[l], p, comp_name, s));
   }
   // the levels left are small ones (the totals halve from level to level): whole subtrees
   if (l < levels) {

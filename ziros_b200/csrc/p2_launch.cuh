@@ -1,5 +1,7 @@
 // p2_launch.cuh — launches of the tensor-core hashing kernels (p2_tensor.cu).
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "fri_fold.cuh"
 #include "matlist.cuh"
@@ -39,4 +41,38 @@ int permute(uint32_t *states, uint64_t n, const P2Params<BabyBear, 16> &p, cudaS
 int wait_errors(uint32_t *count);
 
 }  // namespace p2t
+
+// The same for Goldilocks, widths 12 and 16 (p2_tensor_gl.cu).
+namespace p2g {
+
+template <int W>
+bool takes(const P2Params<Goldilocks, W> &p, uint64_t rows);
+template <int W>
+int hash_rows(const MatList &ml, uint64_t height, uint64_t *digests, const P2Params<Goldilocks, W> &p, const char *name,
+              cudaStream_t s);
+template <int W>
+int compress(const uint64_t *prev, uint64_t *next, uint64_t n_out, const uint64_t *inj, uint64_t inj_h,
+             const P2Params<Goldilocks, W> &p, const char *name, cudaStream_t s);
+template <int W>
+int mt_leaf(const mt::LeafJob *d_jobs, int n, uint64_t tiles, uint64_t perms, const P2Params<Goldilocks, W> &p,
+            const char *name, cudaStream_t s);
+template <int W>
+int mt_compress(const mt::CompJob *d_jobs, int n, uint64_t total, const P2Params<Goldilocks, W> &p, const char *name,
+                cudaStream_t s);
+template <int W>
+int permute(uint64_t *states, uint64_t n, const P2Params<Goldilocks, W> &p, cudaStream_t s);
+int wait_errors(uint32_t *count);
+
+}  // namespace p2g
+
+// ---- the form of a launch, chosen by its size (rows, compressions or states) ----
+// The tensor-core form above its smallest size.
+template <class F, int W>
+bool tensor_takes(const P2Params<F, W> &p, uint64_t rows) {
+  if constexpr (std::is_same<F, BabyBear>::value)
+    return p2t::takes(p, rows);
+  else
+    return p2g::takes<W>(p, rows);
+}
+
 }  // namespace zkb

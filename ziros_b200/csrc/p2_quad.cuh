@@ -422,15 +422,6 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// Largest launch (rows, compressions or states) that takes this form.  BabyBear: every one below
-// the tensor-core form's sizes (p2_tensor.cu).  Goldilocks, against one state per thread: width 16
-// 16,384 rows x 32 columns 216 us against 331, 32,768 359 against 402, 65,536 686 against 664; width 12
-// 16,384 224 against 254, 32,768 371 against 311.
-template <class F, int W>
-constexpr bool takes(uint64_t rows) {
-  return std::is_same<F, BabyBear>::value || rows <= (W == 16 ? 32768 : 16384);
-}
-
 inline unsigned grid_of(uint64_t items, unsigned threads) { return grid_for(items * 4, threads, 1u << 30); }
 
 // Levels per launch for a run of `total` levels: as few launches as MAX_RUN - 1 levels each allow, of

@@ -22,9 +22,11 @@
 #pragma once
 #include "field.cuh"
 #include "poseidon2.cuh"
+#include "tcgen05.cuh"
 
 namespace zkb {
 namespace p2t {
+using namespace tc;
 
 constexpr int NF = 8, NP = 13;   // rounds this form is built for (R_F, R_P)
 constexpr int GROUP = 128;       // threads (= permutations) of one product
@@ -232,24 +234,16 @@ __host__ __device__ constexpr int smem_tables(Mode m) {
 // TMEM address, the image's mbarrier and one per group follow the tables.
 __host__ __device__ constexpr int smem_bytes(Mode m) { return smem_tables(m) + 16 + 8 * MAX_GROUPS; }
 
-// A part of the image, copied by one untiled bulk copy of this GPU's own memory.
-__device__ __forceinline__ void copy_tables(uint32_t dst, int src, int bytes, uint32_t mbar) {
-  asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(__cvta_generic_to_global(kImage.b + src)), "r"((uint32_t)bytes), "r"(mbar)
-               : "memory");
-}
 // The matrices a kernel needs: issued by one thread, completed on mbar.
 __device__ __forceinline__ void copy_image(uint32_t sm, Mode mode, int last_rem, uint32_t mbar) {
   const bool sponge = mode == SPONGE || mode == SPONGE_ANY;
   const int fin = mode == PERM16 ? 2 * SLAB64 : SLAB64, in = sponge ? ABS_BYTES : 2 * SLAB64;
   const int last = mode == SPONGE_ANY ? 7 * ABS_BYTES : mode == SPONGE && last_rem != 8 ? ABS_BYTES : 0;
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar),
-               "r"((uint32_t)(COMMON + fin + in + last))
-               : "memory");
-  copy_tables(sm, 0, COMMON, mbar);
-  copy_tables(sm + S_FIN, mode == PERM16 ? I_FIN16 : I_FIN8, fin, mbar);
-  copy_tables(sm + S_IN, sponge ? I_ABS : I_IN16, in, mbar);
-  if (last) copy_tables(sm + S_LAST, I_ABS + (mode == SPONGE_ANY ? 1 : last_rem) * ABS_BYTES, last, mbar);
+  expect_bytes(mbar, COMMON + fin + in + last);
+  bulk_copy(sm, kImage.b, COMMON, mbar);
+  bulk_copy(sm + S_FIN, kImage.b + (mode == PERM16 ? I_FIN16 : I_FIN8), fin, mbar);
+  bulk_copy(sm + S_IN, kImage.b + (sponge ? I_ABS : I_IN16), in, mbar);
+  if (last) bulk_copy(sm + S_LAST, kImage.b + I_ABS + (mode == SPONGE_ANY ? 1 : last_rem) * ABS_BYTES, last, mbar);
 }
 // The round constants: byte 4 * (W_ONE - 8) of the second W slab meets the constant one.
 __device__ __forceinline__ void put_constants(uint8_t *sm, const P2Params<BabyBear, 16> &p) {
@@ -269,62 +263,6 @@ __device__ __forceinline__ void put_constants(uint8_t *sm, const P2Params<BabyBe
 #pragma unroll
     for (int l = 0; l < 4; l++) sm[base + slot(64, 4 * i + acc_col(l), kb)] = (uint8_t)(v >> (8 * l));
   }
-}
-
-// ------------------------------------------------------------------- PTX wrappers
-// s32 accumulators, u8 x u8, both operands K-major, M = 128.
-__device__ __forceinline__ constexpr uint32_t idesc(int N) {
-  return (2u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(GROUP >> 4) << 24);
-}
-// Shared-memory operand without swizzle: 8 x 16-byte core matrices, 128 bytes apart along N and
-// (N / 8) * 128 bytes apart along K.
-__device__ __forceinline__ uint64_t bdesc(uint32_t addr, int N) {
-  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((N / 8) * 128 / 16) << 16) | ((uint64_t)(128 / 16) << 32) |
-         (1ull << 46);
-}
-// Issued by a whole warp with warp-uniform operands; `one` is set in a single lane.
-__device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint64_t b, uint32_t id, bool acc, uint32_t one) {
-  asm volatile(
-      "{\n\t.reg .pred p, e;\n\tsetp.ne.u32 p, %4, 0;\n\tsetp.ne.u32 e, %5, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-      "r"(a), "l"(b), "r"(id), "r"((uint32_t)acc), "r"(one)
-      : "memory");
-}
-__device__ __forceinline__ void st8(uint32_t a, const uint32_t *v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(a), "r"(v[0]), "r"(v[1]),
-               "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-__device__ __forceinline__ void st4(uint32_t a, const uint32_t *v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v[0]), "r"(v[1]), "r"(v[2]),
-               "r"(v[3])
-               : "memory");
-}
-__device__ __forceinline__ void st1(uint32_t a, uint32_t v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(a), "r"(v) : "memory");
-}
-__device__ __forceinline__ void ld16(uint32_t (&v)[16], uint32_t a) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(a)
-      : "memory");
-}
-// The low 16 bits of 32 columns, two adjacent columns to a register.
-__device__ __forceinline__ void ld16_pack(uint32_t (&v)[16], uint32_t a) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(a)
-      : "memory");
-}
-// Waits for the loads; the registers pass through so that no use moves above the wait.
-__device__ __forceinline__ void ld_wait(uint32_t (&v)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
 }
 
 // --------------------------------------------------------------------- arithmetic
@@ -365,62 +303,6 @@ __device__ __forceinline__ int recombine_small(uint32_t p02, uint32_t p13) {
   const float k = (float)(16777216.0 / 2013265921.0 * (1.0 - 0.00146));
   const float q = __fmaf_rn(f, k, 12582912.0f - 273.0f);
   return (int)(t - __float_as_uint(q) * P);
-}
-
-// ------------------------------------------------------------------------- a group
-struct Group {
-  uint32_t sm;      // shared address of the tables
-  uint32_t tm;      // TMEM address of the group's columns
-  uint32_t tw;      // the same with this warp's lane base (ld / st)
-  uint32_t mbar;    // shared address of the group's mbarrier
-  uint32_t phase;
-  int bar;          // named barrier of the group
-  bool lead;        // this is the warp that issues the products (warp-uniform)
-  uint32_t one;     // set in one lane of it
-  uint32_t polls;   // limit of a wait (0 once one has run out)
-  uint32_t *err;
-};
-
-constexpr uint32_t WAIT_POLLS = 1u << 16;
-
-__device__ __forceinline__ void mma_slab(const Group &g, int d_col, int a_col, int off, int N, bool acc) {
-  mma(g.tm + d_col, g.tm + a_col, bdesc(g.sm + off, N), idesc(N), acc, g.one);
-}
-
-__device__ __forceinline__ bool wait_parity(uint32_t mbar, uint32_t parity, uint32_t polls) {
-  uint32_t done = 0;
-  for (uint32_t n = 0; n < polls && !done; n++) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(mbar), "r"(parity)
-        : "memory");
-  }
-  return done != 0;
-}
-
-// Before the products: this thread's operand stores are complete and its accumulator loads done.
-__device__ __forceinline__ void arrive(const Group &g) {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  asm volatile("bar.sync %0, 128;" ::"r"(g.bar) : "memory");
-  if (g.lead) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// After the products have been issued by the lead thread: everyone waits for them (bounded: a
-// wait that runs out records itself and the group goes on, so every block ends).
-__device__ __forceinline__ void finish(Group &g) {
-  if (g.lead)
-    asm volatile(
-        "{\n\t.reg .pred e;\n\tsetp.ne.u32 e, %1, 0;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(g.mbar),
-        "r"(g.one)
-        : "memory");
-  if (!wait_parity(g.mbar, g.phase, g.polls)) {
-    if (g.polls) atomicAdd(g.err, 1u);
-    g.polls = 0;
-  }
-  g.phase ^= 1;
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
 // One layer's outputs to S-box outputs: 16 words, each x^7 + p in (0, 2p), stored as the next
@@ -556,7 +438,7 @@ __device__ __forceinline__ void rounds(Group &g) {
 
 // The last S-box outputs, as `rounds` left them.
 __device__ __forceinline__ void load_z(const Group &g, uint32_t (&z)[16]) {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+  st_wait();
   ld16(z, g.tw + COL_Z);
   ld_wait(z);
 }
@@ -618,54 +500,32 @@ __device__ __forceinline__ Group setup(uint8_t *sm, const P2Params<BabyBear, 16>
   const uint32_t tables = ctrl + 8;  // mbarrier of the image copies
   const int groups = blockDim.x / GROUP;
   if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tables) : "memory");
-    for (int i = 0; i < groups; i++)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ctrl + 16 + 8 * i) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    init_barrier(tables);
+    for (int i = 0; i < groups; i++) init_barrier(ctrl + 16 + 8 * i);
+    init_fence();
     copy_image(base, mode, last_rem, tables);
   }
   for (int t = threadIdx.x; t < 8 * SLAB64 / 16; t += blockDim.x)
     reinterpret_cast<uint4 *>(sm + S_C)[t] = make_uint4(0, 0, 0, 0);
-  if (threadIdx.x < 32) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ctrl),
-                 "r"(tmem_cols(groups))
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (threadIdx.x < 32) tmem_alloc(ctrl, tmem_cols(groups));
   __syncthreads();
   if (!wait_parity(tables, 0, WAIT_POLLS)) atomicAdd(err, 1u);
   put_constants(sm, p);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  fence_before();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  // warp-uniform by construction; the shuffles let the compiler keep them in uniform registers
-  const int warp = __shfl_sync(0xFFFFFFFFu, (int)threadIdx.x / 32, 0), gi = warp / 4;
-  Group g;
-  g.sm = base;
-  g.tm = __shfl_sync(0xFFFFFFFFu, *reinterpret_cast<volatile uint32_t *>(sm + smem_tables(mode)), 0) + gi * COLS;
-  g.tw = g.tm + ((warp % 4) << 21);
-  g.mbar = ctrl + 16 + 8 * gi;
-  g.phase = 0;
-  g.bar = 1 + gi;
-  g.lead = warp % 4 == 0;
-  g.one = threadIdx.x % GROUP == 0;
-  g.polls = WAIT_POLLS;
-  g.err = err;
+  fence_after();
+  const Group g = make_group(sm, smem_tables(mode), ctrl + 16, COLS, err);
   st1(g.tw + COL_W + W_ONE, 1);
   return g;
 }
 __device__ __forceinline__ void teardown(uint8_t *sm, Mode mode) {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  st_wait();
+  fence_before();
   __syncthreads();
   if (threadIdx.x < 32) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(
-                     *reinterpret_cast<volatile uint32_t *>(sm + smem_tables(mode))),
-                 "r"(tmem_cols(blockDim.x / GROUP))
-                 : "memory");
+    fence_after();
+    tmem_free(*reinterpret_cast<volatile uint32_t *>(sm + smem_tables(mode)), tmem_cols(blockDim.x / GROUP));
   }
 }
 #endif  // __CUDACC__

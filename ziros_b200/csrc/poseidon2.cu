@@ -25,8 +25,8 @@ bool build_p2_params(const uint64_t *rc, size_t n_rc, int rounds_f, int rounds_p
   p->out = out;
   p->rate = 8;
   p->diag_kind = 0;
-  if (sizeof(typename F::T) == 4 && W == 16) {
-    std::vector<uint64_t> v = p2_diagonal(FIELD_BABYBEAR, 16);
+  {
+    const std::vector<uint64_t> v = p2_diagonal(sizeof(typename F::T) == 4 ? FIELD_BABYBEAR : FIELD_GOLDILOCKS, W);
     bool same = true;
     for (int i = 0; i < W; i++) same = same && diag[i] == v[i];
     p->diag_kind = same ? 1 : 0;
@@ -42,38 +42,17 @@ bool build_p2_params(const HasherSpec &h, P2Params<F, W> *p) {
 }
 
 template <class F, int W>
-__global__ void __launch_bounds__(128)
-    p2_batch_kernel(typename F::T *__restrict__ states, size_t n,
-                    const __grid_constant__ P2Params<F, W> p) {
-  using T = typename F::T;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    T s[W];
-    T *g = states + i * W;
-#pragma unroll
-    for (int k = 0; k < W; k++) s[k] = Dom<F>::enter(g[k]);
-    p2_permute<F, W>(s, p);
-#pragma unroll
-    for (int k = 0; k < W; k++) g[k] = Dom<F>::leave(s[k]);
-  }
-}
-
-template <class F, int W>
 int p2_permute_batch(typename F::T *d_states, size_t n_states, const P2Params<F, W> &p,
                      cudaStream_t s) {
   if (n_states == 0) return ZKB_OK;
-  if constexpr (std::is_same<F, BabyBear>::value && W == 16) {
-    if (p2t::takes(p, n_states)) return p2t::permute(d_states, n_states, p, s);
+  if (tensor_takes<F, W>(p, n_states)) {
+    if constexpr (std::is_same<F, BabyBear>::value)
+      return p2t::permute(d_states, n_states, p, s);
+    else
+      return p2g::permute<W>(d_states, n_states, p, s);
   }
-  DeviceContext *ctx;
-  ZKB_TRY(current_context(&ctx));
   const unsigned threads = 128;
-  if (quad::takes<F, W>(n_states)) {
-    ZKB_LAUNCH("p2_permute", s, quad::states_kernel<F, W><<<quad::grid_of(n_states, threads), threads, 0, s>>>(d_states, n_states, p));
-  } else if constexpr (!std::is_same<F, BabyBear>::value) {
-    const unsigned grid = grid_for(n_states, threads, (unsigned)ctx->sm_count * 16u);
-    ZKB_LAUNCH("p2_permute", s, p2_batch_kernel<F, W><<<grid, threads, 0, s>>>(d_states, n_states, p));
-  }
+  ZKB_LAUNCH("p2_permute", s, quad::states_kernel<F, W><<<quad::grid_of(n_states, threads), threads, 0, s>>>(d_states, n_states, p));
   ZKB_CHECK_LAUNCH();
   return ZKB_OK;
 }
