@@ -29,8 +29,9 @@ namespace zkb {
 struct PassGeom {
   int L;                     // log2 of each transform
   int lo;                    // lowest index bit of this pass
-  uint32_t width;            // matrix columns
-  uint32_t chunks_per_row;   // width / C
+  uint32_t width;            // row stride of the matrix
+  uint32_t cols;             // columns from the pointers on (the last chunk may have fewer than C)
+  uint32_t chunks_per_row;   // ceil(cols / C)
   uint32_t groups;           // 2^(L-K) groups per transform
   uint64_t block_stride;     // elements between transforms
   int twist;
@@ -237,6 +238,9 @@ __device__ __forceinline__ void ntt_pass_tile(const typename F::T *in, typename 
     else if (post_scale)
       tw_out[e] = tw_stage<F>(post_scale);
   }
+  // A thread whose column lies past the matrix has done its share of the staging (the barriers
+  // below count the threads that have not exited).
+  if (!PERSIST && chunk * C + c >= g.cols) return;
 
   const size_t col0 = (size_t)blk * g.block_stride + (size_t)chunk * C + c;
   const size_t rs = (size_t)g.width << g.lo;  // elements between consecutive tile rows
@@ -315,8 +319,9 @@ constexpr size_t pass_tile_smem() {
 // needs, so the coefficient matrix never goes back to HBM and no expand pass runs.
 struct FusedGeom {
   int L;
-  uint32_t width;
-  uint32_t chunks_per_row;
+  uint32_t width;           // row stride
+  uint32_t cols;            // columns from the pointers on
+  uint32_t chunks_per_row;  // ceil(cols / C)
   uint32_t blocks;   // 2^(L-K)
   int log_b;
   uint64_t n;        // 2^L
@@ -349,6 +354,7 @@ __device__ __forceinline__ void lde_fused_tile(const typename F::T *in, typename
   const uint32_t m_lo = lm ? (__brev(B) >> (32 - lm)) : 0u;
   const uint32_t c = threadIdx.x % C;
   const uint32_t i = threadIdx.x / C;
+  const bool col_ok = chunk * C + c < g.cols;
 
   for (uint32_t e = threadIdx.x; e < (1u << K); e += blockDim.x) {
     const uint32_t ii = e / R1, tt = e % R1;
@@ -378,7 +384,7 @@ __device__ __forceinline__ void lde_fused_tile(const typename F::T *in, typename
           if constexpr (PERSIST)
             x[j] = __ldcg(p);
           else
-            x[j] = *p;
+            x[j] = col_ok ? *p : 0;
           p += step;
         }
       }
@@ -432,7 +438,7 @@ __device__ __forceinline__ void lde_fused_tile(const typename F::T *in, typename
       });
     }
     __syncthreads();
-    if (active) {
+    if (active && (PERSIST || col_ok)) {
       const uint32_t r = g.log_b ? (__brev((uint32_t)jc) >> (32 - g.log_b)) : 0u;
       T *blk = out + (uint64_t)r * g.n * g.width + colc + (size_t)m_lo * g.width;
 #pragma unroll 1

@@ -465,6 +465,7 @@ int PersistPlan::build(const std::vector<PersistTrace> &traces, int log_b, const
         st.pg.L = L;
         st.pg.lo = lo;
         st.pg.width = w;
+        st.pg.cols = cols;
         st.pg.chunks_per_row = cols / C;
         st.pg.groups = 1u << (L - K);
         st.pg.block_stride = (uint64_t)w << L;
@@ -503,6 +504,7 @@ int PersistPlan::build(const std::vector<PersistTrace> &traces, int log_b, const
         st.dep = prev;
         st.fg.L = L;
         st.fg.width = w;
+        st.fg.cols = cols;
         st.fg.chunks_per_row = cols / C;
         st.fg.blocks = 1u << (L - Kf);
         st.fg.log_b = log_b;
