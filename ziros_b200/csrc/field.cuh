@@ -164,6 +164,53 @@ struct Goldilocks {
     if (r < t1) r += EPS;
     return canon(r);
   }
+#ifdef __CUDACC__
+  // r0 + r1 2^32 + r2 2^64 + r3 2^96 mod p, some 64-bit representative: 2^64 = 2^32 - 1 and 2^96 = -1, so
+  // the value is (r1 + r2) 2^32 + r0 - r2 - r3 = x + k 2^64 with k in {-1, 0, 1}, and x + k (2^32 - 1)
+  // neither overflows nor goes below zero.
+  __device__ __forceinline__ static uint64_t fold(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    uint32_t l, h;
+    asm("{\n\t.reg .u32 a0, a1, k, m;\n\t"
+        "add.cc.u32 a1, %3, %4;\n\taddc.u32 k, 0, 0;\n\t"
+        "sub.cc.u32 a0, %2, %4;\n\tsubc.cc.u32 a1, a1, 0;\n\tsubc.u32 k, k, 0;\n\t"
+        "sub.cc.u32 a0, a0, %5;\n\tsubc.cc.u32 a1, a1, 0;\n\tsubc.u32 k, k, 0;\n\t"
+        "shr.s32 m, k, 31;\n\t"
+        "sub.cc.u32 %0, a0, k;\n\tsubc.u32 a1, a1, m;\n\tadd.u32 %1, a1, k;\n\t}"
+        : "=r"(l), "=r"(h)
+        : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
+    return ((uint64_t)h << 32) | l;
+  }
+  // a * b (+ y), any 64-bit operands, some 64-bit representative of the result: a 128-bit product from
+  // four 32x32 partial products (eight 32-bit multiplies, one carry chain) and its fold.  38 cycles of an
+  // SM sub-partition per warp; `mul` below 47 (with this fold and a canonical result the NTT passes took
+  // 0.8 % longer), with wide products (mul.wide) 43 to 49.
+  template <bool ADD = false>
+  __device__ __forceinline__ static uint64_t mul_any(uint64_t a, uint64_t b, uint64_t y = 0) {
+    uint32_t r0, r1, r2, r3;
+    const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
+    asm("mul.lo.u32 %0, %4, %6;\n\t"
+        "mul.hi.u32 %1, %4, %6;\n\t"
+        "mad.lo.cc.u32 %1, %4, %7, %1;\n\t"
+        "madc.hi.u32 %2, %4, %7, 0;\n\t"
+        "mad.lo.cc.u32 %1, %5, %6, %1;\n\t"
+        "madc.hi.cc.u32 %2, %5, %6, %2;\n\t"
+        "madc.hi.u32 %3, %5, %7, 0;\n\t"
+        "mad.lo.cc.u32 %2, %5, %7, %2;\n\t"
+        "addc.u32 %3, %3, 0;"
+        : "=&r"(r0), "=&r"(r1), "=&r"(r2), "=&r"(r3)
+        : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
+    if constexpr (ADD)  // (2^64 - 1)^2 + 2^64 - 1 < 2^128
+      asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, 0;\n\taddc.u32 %3, %3, 0;"
+          : "+r"(r0), "+r"(r1), "+r"(r2), "+r"(r3)
+          : "r"((uint32_t)y), "r"((uint32_t)(y >> 32)));
+    return fold(r0, r1, r2, r3);
+  }
+  // x^7 of any 64-bit operand, some 64-bit representative.
+  __device__ __forceinline__ static uint64_t pow7_any(uint64_t x) {
+    const uint64_t x2 = mul_any(x, x), x3 = mul_any(x2, x), x4 = mul_any(x2, x2);
+    return mul_any(x3, x4);
+  }
+#endif
   __host__ __device__ __forceinline__ static uint64_t mul(uint64_t a, uint64_t b) {
 #ifdef __CUDA_ARCH__
     // 128-bit product from four 32x32 partial products (eight 32-bit multiplies, one

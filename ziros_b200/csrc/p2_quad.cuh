@@ -45,7 +45,7 @@ template <>
 struct Ops<Goldilocks> {
   using T = unsigned long long;
   static __host__ __device__ T rc(T c) { return c; }
-  static __device__ __forceinline__ T sbox(T x, T c) { return p2_sbox<Goldilocks>(Goldilocks::add(x, c)); }
+  static __device__ __forceinline__ T sbox(T x, T c) { return Goldilocks::canon(Goldilocks::pow7_any(Goldilocks::add(x, c))); }
   static __device__ __forceinline__ T mul(T a, T b) { return Goldilocks::mul(a, b); }
   static __device__ __forceinline__ T next_y(T, T w, T sum, T d0) { return Goldilocks::add(Goldilocks::mul(w, d0), sum); }
 };
@@ -152,6 +152,64 @@ __device__ __forceinline__ void permute(typename F::T (&s)[4], const Consts<F> &
     }
     if (q == 0) s[0] = y;
   }
+}
+
+// The same with one word to a lane, sixteen lanes a state (width 12: the last four idle), for the upper tree
+// levels, where threads are left over: one S-box deep instead of four, at two
+// and a half times the instructions per state.  d: this lane's diagonal word.
+template <class F, int W>
+__device__ __forceinline__ typename F::T ext_mds_lane(typename F::T s, int lane) {
+  using D = Dom<F>;
+  using T = typename F::T;
+  using U = typename Ops<F>::T;
+  const T next = (T)__shfl_sync(0xFFFFFFFFu, (U)s, (lane & ~3) | ((lane + 1) & 3), 16);
+  T t = D::add(s, (T)__shfl_xor_sync(0xFFFFFFFFu, (U)s, 1));
+  t = D::add(t, (T)__shfl_xor_sync(0xFFFFFFFFu, (U)t, 2));
+  const T y = D::add(t, D::add(s, D::add(next, next)));
+  T c = D::add(y, (T)__shfl_xor_sync(0xFFFFFFFFu, (U)y, 4));
+  c = D::add(c, (T)__shfl_xor_sync(0xFFFFFFFFu, (U)c, 8));
+  return W == 12 && lane >= 12 ? 0 : D::add(y, c);
+}
+template <class F, int W>
+__device__ __forceinline__ typename F::T permute_lane(typename F::T s, const Consts<F> &k, int lane) {
+  using D = Dom<F>;
+  using T = typename F::T;
+  using U = typename Ops<F>::T;
+  const int half = k.half, partial = k.partial;
+  const T d = k.diag[lane];
+  T rc = k.full[lane];
+  s = ext_mds_lane<F, W>(s, lane);
+#pragma unroll 1
+  for (int h = 0; h < 2; h++) {
+#pragma unroll 1
+    for (int r = 0; r < half; r++) {
+      const T nx = k.full[min(h * half + r + 1, 2 * half - 1) * 16 + lane];
+      s = Ops<F>::sbox(s, rc);
+      if (W == 12 && lane >= 12) s = 0;
+      s = ext_mds_lane<F, W>(s, lane);
+      rc = nx;
+    }
+    if (h) break;
+    T c = k.part[0], y = s;
+#pragma unroll 1
+    for (int pr = 0; pr < partial; pr++) {
+      const T cn = k.part[min(pr + 1, partial - 1)];
+      T rest = lane ? s : 0;
+      const T m = Ops<F>::mul(s, d);
+      rest = D::add(rest, (T)__shfl_xor_sync(0xFFFFFFFFu, (U)rest, 1));
+      const T w0 = Ops<F>::sbox(y, c);
+      rest = D::add(rest, (T)__shfl_xor_sync(0xFFFFFFFFu, (U)rest, 2));
+      rest = D::add(rest, (T)__shfl_xor_sync(0xFFFFFFFFu, (U)rest, 4));
+      rest = D::add(rest, (T)__shfl_xor_sync(0xFFFFFFFFu, (U)rest, 8));
+      const T w = (T)__shfl_sync(0xFFFFFFFFu, (U)w0, 0, 16), sum = D::add(rest, w);
+      y = Ops<F>::next_y(rest, w0, sum, d);
+      s = D::add(m, sum);
+      if (W == 12 && lane >= 12) s = 0;
+      c = cn;
+    }
+    if (lane == 0) s = y;
+  }
+  return s;
 }
 
 template <class T>
@@ -314,6 +372,30 @@ __device__ __forceinline__ void subtree(uint64_t block, int levels, Layer layer,
   T *from = buf, *to = buf;  // level j's digests: 2^(levels - 1 - j) of them, one after another
   for (int j = 0; j < levels; j++) {
     const uint64_t cnt = 1ull << (levels - 1 - j), base = block * cnt, below = nodes(j), n = nodes(j + 1);
+    if (cnt * 16 <= blockDim.x) {  // few enough for a lane to a word
+      const int lane = threadIdx.x & 15;
+      const uint64_t o = threadIdx.x / 16;
+      const bool live = o < cnt && base + o < n;
+      if (threadIdx.x / 32 * 2 < cnt) {  // whole warps
+        T s = 0;
+        const int child = lane / OUT;
+        if (live && child < 2) {
+          if (j == 0)
+            s = layer(0)[(base + o) * 2 * OUT + lane];
+          else if (2 * (base + o) + child < below)
+            s = from[o * 2 * OUT + lane];
+        }
+        s = Dom<F>::leave(permute_lane<F, W>(Dom<F>::enter(s), k, lane));
+        if (live && lane < OUT) {
+          layer(j + 1)[(base + o) * OUT + lane] = s;
+          if (j + 1 < levels) to[o * OUT + lane] = s;
+        }
+      }
+      __syncthreads();
+      from = to;
+      to += cnt * OUT;
+      continue;
+    }
     for (uint64_t w = threadIdx.x / 32 * 8; w < cnt && base + w < n; w += blockDim.x >> 2) {
       const uint64_t o = w + threadIdx.x % 32 / 4;
       const bool live = o < cnt && base + o < n;
@@ -430,7 +512,8 @@ inline int run_levels(int total) {
   const int stages = (total + MAX_RUN - 2) / (MAX_RUN - 1);
   return (total + stages - 1) / stages;
 }
-inline unsigned run_threads(int levels) {  // four threads for each of the first level's nodes
+// Four threads for each of the first level's nodes, and sixteen for each of its fourth's.
+inline unsigned run_threads(int levels) {
   const int t = 4 << (levels - 1);
   return (unsigned)(t < 32 ? 32 : t > 512 ? 512 : t);
 }

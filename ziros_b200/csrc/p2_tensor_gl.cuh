@@ -186,49 +186,6 @@ __device__ __forceinline__ void put_constants(uint8_t *sm, const P2Params<Goldil
 }
 
 // --------------------------------------------------------------------- arithmetic
-// r0 + r1 2^32 + r2 2^64 + r3 2^96 mod p, some 64-bit representative: 2^64 = 2^32 - 1 and 2^96 = -1, so the
-// value is (r1 + r2) 2^32 + r0 - r2 - r3 = x + k 2^64 with k in {-1, 0, 1}, and x + k (2^32 - 1) neither
-// overflows nor goes below zero.
-__device__ __forceinline__ uint64_t fold(uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
-  uint32_t l, h;
-  asm("{\n\t.reg .u32 a0, a1, k, m;\n\t"
-      "add.cc.u32 a1, %3, %4;\n\taddc.u32 k, 0, 0;\n\t"
-      "sub.cc.u32 a0, %2, %4;\n\tsubc.cc.u32 a1, a1, 0;\n\tsubc.u32 k, k, 0;\n\t"
-      "sub.cc.u32 a0, a0, %5;\n\tsubc.cc.u32 a1, a1, 0;\n\tsubc.u32 k, k, 0;\n\t"
-      "shr.s32 m, k, 31;\n\t"
-      "sub.cc.u32 %0, a0, k;\n\tsubc.u32 a1, a1, m;\n\tadd.u32 %1, a1, k;\n\t}"
-      : "=r"(l), "=r"(h)
-      : "r"(r0), "r"(r1), "r"(r2), "r"(r3));
-  return ((uint64_t)h << 32) | l;
-}
-// S-box with this product and reduction 137 cycles of an SM sub-partition per warp; with canonical results
-// after each product (Goldilocks::mul) 174, with wide products (mul.wide) 147 to 165.
-// a * b (+ y), any 64-bit operands, some 64-bit representative of the result.
-template <bool ADD>
-__device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b, uint64_t y = 0) {
-  uint32_t r0, r1, r2, r3;
-  const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
-  asm("mul.lo.u32 %0, %4, %6;\n\t"
-      "mul.hi.u32 %1, %4, %6;\n\t"
-      "mad.lo.cc.u32 %1, %4, %7, %1;\n\t"
-      "madc.hi.u32 %2, %4, %7, 0;\n\t"
-      "mad.lo.cc.u32 %1, %5, %6, %1;\n\t"
-      "madc.hi.cc.u32 %2, %5, %6, %2;\n\t"
-      "madc.hi.u32 %3, %5, %7, 0;\n\t"
-      "mad.lo.cc.u32 %2, %5, %7, %2;\n\t"
-      "addc.u32 %3, %3, 0;"
-      : "=&r"(r0), "=&r"(r1), "=&r"(r2), "=&r"(r3)
-      : "r"(a0), "r"(a1), "r"(b0), "r"(b1));
-  if constexpr (ADD)  // (2^64 - 1)^2 + 2^64 - 1 < 2^128
-    asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, 0;\n\taddc.u32 %3, %3, 0;"
-        : "+r"(r0), "+r"(r1), "+r"(r2), "+r"(r3)
-        : "r"((uint32_t)y), "r"((uint32_t)(y >> 32)));
-  return fold(r0, r1, r2, r3);
-}
-__device__ __forceinline__ uint64_t sbox(uint64_t x) {
-  const uint64_t x2 = mul<false>(x, x), x3 = mul<false>(x2, x), x4 = mul<false>(x2, x2);
-  return mul<false>(x3, x4);
-}
 // e + f 2^32 for e, f < 2^56, some 64-bit representative: f = f0 + f1 2^32 adds (f0 + f1) 2^32 - f1.
 __device__ __forceinline__ uint64_t join(uint32_t e0, uint32_t e1, uint32_t f0, uint32_t f1) {
   uint32_t l, h;
@@ -288,7 +245,7 @@ __device__ __forceinline__ void full_sbox(const Group &g) {
     uint64_t z[4];
     load_outputs<SMALL>(z, g.tw + S::COL_D + 32 * c);
 #pragma unroll
-    for (int e = 0; e < 4; e++) z[e] = sbox(z[e]);
+    for (int e = 0; e < 4; e++) z[e] = Goldilocks::pow7_any(z[e]);
     store_words(g.tw + S::COL_Z + 8 * c, z);
   }
 }
@@ -334,11 +291,12 @@ __device__ __forceinline__ void rounds(Group &g) {
     uint64_t w[4];
     load_outputs<false>(w, g.tw + S::COL_D);
     const uint64_t c0 = kImage<W>.c[0], c1 = kImage<W>.c[1], c2 = kImage<W>.c[2];
-    w[0] = sbox(w[0]);
-    w[1] = sbox(mul<true>(c0, w[0], w[1]));
+    using G = Goldilocks;
+    w[0] = G::pow7_any(w[0]);
+    w[1] = G::pow7_any(G::mul_any<true>(c0, w[0], w[1]));
     if (i + 1 < BLOCKS) {  // the last block has two rounds
-      w[2] = sbox(mul<true>(c0, w[1], mul<true>(c1, w[0], w[2])));
-      w[3] = sbox(mul<true>(c0, w[2], mul<true>(c1, w[1], mul<true>(c2, w[0], w[3]))));
+      w[2] = G::pow7_any(G::mul_any<true>(c0, w[1], G::mul_any<true>(c1, w[0], w[2])));
+      w[3] = G::pow7_any(G::mul_any<true>(c0, w[2], G::mul_any<true>(c1, w[1], G::mul_any<true>(c2, w[0], w[3]))));
       store_words(g.tw + S::COL_W + 8 * i, w);
     } else {
       const uint32_t v[4] = {(uint32_t)w[0], (uint32_t)(w[0] >> 32), (uint32_t)w[1], (uint32_t)(w[1] >> 32)};
