@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "engine.cuh"
+#include "ntt_tc.cuh"
 #include "p2_launch.cuh"
 
 namespace zkb {
@@ -275,11 +276,12 @@ int zkb_set_ntt_tile_loads(int mode) {
 int zkb_ntt_tile_load_errors(uint32_t *count) {
   ZKB_ENTRY();
   ZKB_REQUIRE(count != nullptr, "null count");
-  uint32_t bb = 0, gl = 0;
+  uint32_t bb = 0, gl = 0, tc = 0;
+  ZKB_TRY(ntt_tc::wait_errors(&tc));
   ZKB_TRY(p2t::wait_errors(&bb));
   ZKB_TRY(p2g::wait_errors(&gl));
   ZKB_TRY(ntt_tma_wait_errors(count));
-  *count += bb + gl;
+  *count += bb + gl + tc;
   return ZKB_OK;
 }
 

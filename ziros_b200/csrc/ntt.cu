@@ -29,6 +29,7 @@
 #include "common.cuh"
 #include "engine.cuh"
 #include "field.cuh"
+#include "ntt_tc.cuh"
 #include "ntt_tile.cuh"
 
 namespace zkb {
@@ -476,6 +477,24 @@ static constexpr int pass_kmax() {
   return sizeof(typename F::T) == 4 ? 10 : 7;
 }
 
+// Smallest Goldilocks pass (in tiles) on the tensor cores: nearly one tile an SM.  2^16 x 30: 100 us with them
+// from 300 tiles on, 142 from 1,480 on; 2^16 x 8 45 from 140 on, 57 from 296 on.
+static constexpr uint64_t NTT_TC_MIN_TILES = 128;
+
+// Largest pass of a default plan over n rows of `width` columns: a Goldilocks pass of 8 bits is slower than
+// one of 7 as butterflies and faster on the tensor cores (2^16 x 30: two passes, 100 us, against
+// three, 142).
+template <class F>
+static int plan_kmax(const void *base, uint64_t n, uint32_t width, uint32_t stride) {
+  if constexpr (sizeof(typename F::T) == 8) {
+    const uint32_t C = ntt_tc::chunk(8), chunks = (width + C - 1) / C;
+    if (n >= 256 && chunks * (n >> 8) >= NTT_TC_MIN_TILES && (chunks * C - width) * 4 <= width &&
+        ntt_tile_loads().load() == 1 && stride % 2 == 0 && ((uintptr_t)base & 15) == 0)
+      return 8;
+  }
+  return pass_kmax<F>();
+}
+
 // Runs the passes `ks` (bit counts, top first) starting at index bit hi_start, over
 // `width` columns of a matrix whose rows are `stride` elements apart (0: width).
 template <class F>
@@ -484,6 +503,7 @@ static int run_plan(const typename F::T *in, typename F::T *out, int L, uint32_t
                     typename F::T last_scale, const std::vector<int> &ks, int hi_start,
                     cudaStream_t s, uint32_t cmax = 0, uint32_t stride = 0) {
   using T = typename F::T;
+  const bool tc = cmax == 0;  // passes on the tensor cores unless a column chunk is asked for
   if (cmax == 0) cmax = sizeof(T) == 4 ? 16 : 8;
   if (stride == 0) stride = width;
   const std::vector<ColSeg> segs = col_segments(width, cmax, n_blocks << L, sizeof(T));
@@ -506,6 +526,22 @@ static int run_plan(const typename F::T *in, typename F::T *out, int L, uint32_t
     }
     const T scale = (pi + 1 == ks.size()) ? last_scale : (T)0;
     int rc = ZKB_OK;
+    if constexpr (sizeof(T) == 8) {
+      const uint32_t C = tc ? ntt_tc::chunk(K) : 0;
+      const uint32_t chunks = C ? (width + C - 1) / C : 0;
+      const uint64_t tiles = (uint64_t)chunks * g.groups * n_blocks;
+      if (C && tiles >= NTT_TC_MIN_TILES && (chunks * C - width) * 4 <= width &&
+          tma_tiles(src, sizeof(T), stride, C, L, g.lo, K, n_blocks, width)) {
+        CUtensorMap map;
+        ZKB_TRY(pass_tensor_map(&map, src, sizeof(T), g, width, K, n_blocks, C));
+        g.cols = width;
+        g.chunks_per_row = chunks;
+        ZKB_TRY(ntt_tc::pass(K, out, g, tiles, tw, inverse, scale, map, s));
+        src = out;
+        hi = g.lo;
+        continue;
+      }
+    }
     for (const ColSeg &sg : segs) {
       const uint32_t C = sg.C;
       const T *sp = src + sg.col0;
@@ -552,7 +588,7 @@ static int run_passes(const typename F::T *in, typename F::T *out, int L, uint32
                       uint64_t n_blocks, const typename F::T *tw, bool inverse,
                       typename F::T last_scale, cudaStream_t s) {
   return run_plan<F>(in, out, L, width, n_blocks, tw, inverse, last_scale,
-                     plan_passes(L, pass_kmax<F>()), L, s);
+                     plan_passes(L, plan_kmax<F>(in, 1ull << L, width, width)), L, s);
 }
 
 // --------------------------------------------------------- fused LDE middle
@@ -759,8 +795,8 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
     ZKB_TRY(lde_tune_check(field_id<F>(), width, *tune));
     tn = *tune;
   }
-  const int kmax = tn.kmax ? tn.kmax : pass_kmax<F>();
   const uint64_t n = 1ull << log_h;
+  const int kmax = tn.kmax ? tn.kmax : plan_kmax<F>(d_trace, n, width, stride);
   const T *ctab;
   ZKB_TRY(get_coset_table<F>(log_h, log_b, shift, &ctab, s));
   if (log_h == 0) {
@@ -792,6 +828,27 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
     g.n = n;
     const T *ctab_t, *ftw_t;
     ZKB_TRY(get_fused_tables<F>(log_h, log_b, shift, Kf, ctab, ftw, &ctab_t, &ftw_t, s));
+    bool fused_done = false;
+    if constexpr (sizeof(T) == 8) {
+      const uint32_t C = tn.c_fused ? 0 : ntt_tc::chunk(Kf);
+      const uint32_t chunks = C ? (width + C - 1) / C : 0;
+      const uint64_t tiles = (uint64_t)chunks * g.blocks;
+      if (C && tiles >= NTT_TC_MIN_TILES && (chunks * C - width) * 4 <= width &&
+          tma_tiles(src, sizeof(T), stride, C, log_h, 0, Kf, 1, width)) {
+        // block B's rows as the tile of a pass at bits [0, K) of one transform
+        PassGeom pg;
+        pg.L = log_h;
+        pg.lo = 0;
+        pg.width = stride;
+        CUtensorMap map;
+        ZKB_TRY(pass_tensor_map(&map, src, sizeof(T), pg, width, Kf, 1, C));
+        g.cols = width;
+        g.chunks_per_row = chunks;
+        ZKB_TRY(ntt_tc::fused(Kf, d_out, g, tiles, itw, ftw, ctab_t, ftw_t, map, s));
+        fused_done = true;
+      }
+    }
+    if (!fused_done)
     for (const ColSeg &sg : col_segments(width, tn.c_fused ? tn.c_fused : 8, n << log_b, sizeof(T))) {
       g.cols = sg.cols;
       g.chunks_per_row = (sg.cols + sg.C - 1) / sg.C;

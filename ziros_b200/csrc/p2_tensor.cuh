@@ -21,6 +21,7 @@
 // next absorb step are one product.
 #pragma once
 #include "field.cuh"
+#include "limbs.cuh"
 #include "poseidon2.cuh"
 #include "tcgen05.cuh"
 
@@ -281,16 +282,10 @@ __device__ __forceinline__ int sbox(int x) {
   const int x4 = smul(x2, x2);
   return smul(x3, x4);
 }
-// The output word of four accumulators, congruent to a0 + a1 2^8 + a2 2^16 + a3 2^24 mod p and in
-// [-p, 1.04 p]: u = a0 + a1 2^8 and v = a2 + a3 2^8 stay below 0.97 p (at most 120 operand
-// bytes, 120 * 255 * 255 * 257 < 2^31); q = floor(v * 139810 / 2^32) is at most the true quotient of
-// v 2^16 by p (2^32 * 2^16 / p = 139810.13) and less than 1.07 below it.
 __device__ __forceinline__ int recombine(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
-  const uint32_t u = a0 + (a1 << 8), v = a2 + (a3 << 8);
-  const uint32_t q = __umulhi(v, 139810u) + 1;
-  return (int)(u + (v << 16) - q * P);
+  return limbs::babybear(a0, a1, a2, a3);
 }
-// The same for the external matrix alone, whose accumulators stay below 2^14 (35 * 255 + 255), read
+// An output of the external matrix alone, whose accumulators stay below 2^14 (35 * 255 + 255), read
 // in pairs as p02 = a0 + a2 2^16 and p13 = a1 + a3 2^16.  The quotient comes from a3 as a float:
 // f = 2^15 + a3 exactly, k = (1 - 0.00146) 2^24 / p, so f k - 273 lies between 0.33 and 0.45 below
 // a3 2^24 / p and the fma rounds it to q in the low mantissa bits, 0x4B400000 + q.  The rest of the

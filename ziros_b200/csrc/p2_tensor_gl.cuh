@@ -9,6 +9,7 @@
 // last product the state.  Round constants ride on a word whose one set byte names the layer.
 #pragma once
 #include "field.cuh"
+#include "limbs.cuh"
 #include "p2_consts.h"
 #include "poseidon2.cuh"
 #include "tcgen05.cuh"
@@ -47,10 +48,7 @@ struct Shape {
   static constexpr int SMEM = CTRL + 16 + 8 * MAX_GROUPS;
 };
 
-// Column of the weight-2^(8 l) accumulator among an output's eight: pairs (0, 2), (1, 3), (4, 6), (5, 7).
-__host__ __device__ constexpr int acc_col(int l) {
-  return (l & 4) | ((l & 3) == 1 ? 2 : (l & 3) == 2 ? 1 : (l & 3));
-}
+__host__ __device__ constexpr int acc_col(int l) { return limbs::goldilocks_col(l); }
 __host__ __device__ constexpr int slot(int N, int n, int k) {
   return ((k >> 4) * (N >> 3) + (n >> 3)) * 128 + (n & 7) * 16 + (k & 15);
 }
@@ -142,6 +140,26 @@ constexpr bool absorb_fits(int w) {
 }
 static_assert(absorb_fits(12) && absorb_fits(16), "the fused absorb layer needs entries below 256");
 
+// The largest sum over a layer's operand bytes of one accumulator column (constants included).
+template <int W>
+constexpr uint32_t max_column() {
+  using S = Shape<W>;
+  const Image<W> m = make_image<W>();
+  uint32_t best = 0;
+  for (int part = 0; part < 2 + BLOCKS; part++) {
+    const int base = part == 0 ? S::O : part == 1 ? S::ABS : S::y_off(part - 2);
+    const int N = part < 2 ? S::N : 32, steps = part == 0 ? S::ZS + S::WS : part == 1 ? S::ZS + 2 : S::ZS + part - 2;
+    for (int n = 0; n < N; n++) {
+      uint32_t sum = 1;  // the constant's byte, against a one
+      for (int k = 0; k < 32 * steps; k++) sum += m.b[base + slot(N, n, k)];
+      best = sum > best ? sum : best;
+    }
+  }
+  return best;
+}
+static_assert(max_column<12>() <= limbs::MAX_COLUMN && max_column<16>() <= limbs::MAX_COLUMN,
+              "accumulators exceed the recombination's range");
+
 template <int W>
 bool usable(const P2Params<Goldilocks, W> &p) {
   return p.diag_kind == 1 && p.rounds_f == NF && p.rounds_p == NP;
@@ -186,30 +204,14 @@ __device__ __forceinline__ void put_constants(uint8_t *sm, const P2Params<Goldil
 }
 
 // --------------------------------------------------------------------- arithmetic
-// e + f 2^32 for e, f < 2^56, some 64-bit representative: f = f0 + f1 2^32 adds (f0 + f1) 2^32 - f1.
-__device__ __forceinline__ uint64_t join(uint32_t e0, uint32_t e1, uint32_t f0, uint32_t f1) {
-  uint32_t l, h;
-  asm("{\n\t.reg .u32 x, k;\n\t"
-      "add.u32 x, %3, %5;\n\t"
-      "sub.cc.u32 %0, %2, %5;\n\tsubc.u32 x, x, 0;\n\t"
-      "add.cc.u32 %1, x, %4;\n\taddc.u32 k, 0, 0;\n\t"
-      "sub.cc.u32 %0, %0, k;\n\tsubc.u32 %1, %1, 0;\n\tadd.u32 %1, %1, k;\n\t}"
-      : "=&r"(l), "=&r"(h)
-      : "r"(e0), "r"(e1), "r"(f0), "r"(f1));
-  return ((uint64_t)h << 32) | l;
-}
 // An output of the external matrix: accumulators below 2^14 (35 * 255 + 255), in pairs a0 + a2 2^16,
 // a1 + a3 2^16, a4 + a6 2^16, a5 + a7 2^16.
 __device__ __forceinline__ uint64_t recombine_small(uint32_t p02, uint32_t p13, uint32_t p46, uint32_t p57) {
   const uint64_t e = p02 + ((uint64_t)p13 << 8), f = p46 + ((uint64_t)p57 << 8);
-  return join((uint32_t)e, (uint32_t)(e >> 32), (uint32_t)f, (uint32_t)(f >> 32));
+  return limbs::goldilocks_join(e, f);
 }
-// An output of any layer: accumulators below 2^25 (at most 312 operand bytes), a in column order.
-__device__ __forceinline__ uint64_t recombine(const uint32_t *a) {
-  const uint64_t e = a[0] + ((uint64_t)a[2] << 8) + ((uint64_t)a[1] << 16) + ((uint64_t)a[3] << 24);
-  const uint64_t f = a[4] + ((uint64_t)a[6] << 8) + ((uint64_t)a[5] << 16) + ((uint64_t)a[7] << 24);
-  return join((uint32_t)e, (uint32_t)(e >> 32), (uint32_t)f, (uint32_t)(f >> 32));
-}
+// An output of any layer.
+__device__ __forceinline__ uint64_t recombine(const uint32_t *a) { return limbs::goldilocks(a); }
 
 __device__ __forceinline__ void store_words(uint32_t col, const uint64_t (&z)[4]) {
   const uint32_t v[8] = {(uint32_t)z[0], (uint32_t)(z[0] >> 32), (uint32_t)z[1], (uint32_t)(z[1] >> 32),
