@@ -678,15 +678,31 @@ static int launch_fused(const typename F::T *in, typename F::T *out, const Fused
 }
 
 // ------------------------------------------------------- auxiliary kernels
-template <class F>
-__global__ void bitrev_rows_kernel(const typename F::T *__restrict__ in, typename F::T *__restrict__ out,
-                                   int L, uint32_t width, uint64_t total) {
-  for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t row = idx / width, c = idx - row * width;
-    uint64_t r = L ? (__brevll(row) >> (64 - L)) : 0;
-    out[r * width + c] = in[idx];
+// out[rev(row)] = in[row].  A block takes BITREV_ROWS consecutive rows, read as one run of elements whose rows
+// come from 32-bit divisions; bound by the writes, runs of one row each.  2^18 x 37 words: 23 us; runs
+// of eight rows on both sides, fewer elements in flight per thread, 39.
+constexpr uint32_t BITREV_ROWS = 32;
+template <class F, class Idx>
+__global__ void __launch_bounds__(256) bitrev_rows_kernel(const typename F::T *__restrict__ in,
+                                                          typename F::T *__restrict__ out, int L, uint32_t width) {
+  const uint64_t row0 = (uint64_t)blockIdx.x * BITREV_ROWS, left = (1ull << L) - row0;
+  const Idx n = (Idx)(left < BITREV_ROWS ? left : BITREV_ROWS) * width;
+  const typename F::T *src = in + row0 * width;
+#pragma unroll 4
+  for (Idx e = threadIdx.x; e < n; e += 256) {
+    const Idx r = e / width, c = e - r * width;
+    const uint64_t to = L ? (__brevll(row0 + r) >> (64 - L)) : 0;
+    out[to * width + c] = src[e];
   }
+}
+template <class F>
+static int bitrev_rows(const typename F::T *in, typename F::T *out, int L, uint32_t width, cudaStream_t s) {
+  const unsigned blocks = (unsigned)(((1ull << L) + BITREV_ROWS - 1) / BITREV_ROWS);
+  if (width < (1u << 26))
+    ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F, uint32_t><<<blocks, 256, 0, s>>>(in, out, L, width));
+  else
+    ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F, uint64_t><<<blocks, 256, 0, s>>>(in, out, L, width));
+  return ZKB_OK;
 }
 
 // Coefficients in bit-reversed row order -> b twisted copies in natural order.
@@ -720,10 +736,7 @@ int ntt_dft_dev(typename F::T *d, int log_h, uint32_t width, bool inverse, cudaS
   T scale = 0;
   if (inverse) scale = Dom<F>::encode(inv_host<F>((T)(n % (uint64_t)F::P)));
   ZKB_TRY(run_passes<F>(d, tmp.as<T>(), log_h, width, 1, tw, inverse, scale, s));
-  ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F><<<grid_for(n * width, 256), 256, 0, s>>>(tmp.as<T>(), d, log_h, width,
-                                                                   n * width));
-  ZKB_CHECK_LAUNCH();
-  return ZKB_OK;
+  return bitrev_rows<F>(tmp.as<T>(), d, log_h, width, s);
 }
 
 template <class F>
@@ -797,6 +810,13 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
   }
   const uint64_t n = 1ull << log_h;
   const int kmax = tn.kmax ? tn.kmax : plan_kmax<F>(d_trace, n, width, stride);
+  // Natural order: the transform goes to scratch, its rows then into the caller's buffer.
+  T *const natural = d_out;
+  ScratchBuf reversed;
+  if (!bitrev) {
+    ZKB_TRY(reversed.alloc((n << log_b) * width * sizeof(T), s));
+    d_out = reversed.as<T>();
+  }
   const T *ctab;
   ZKB_TRY(get_coset_table<F>(log_h, log_b, shift, &ctab, s));
   if (log_h == 0) {
@@ -863,14 +883,7 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
       ZKB_TRY(run_plan<F>(d_out, d_out, log_h, width, 1ull << log_b, ftw, false, (T)0, tail,
                           log_h - Kf, s, tn.c_pass, stride));
   }
-  if (!bitrev) {
-    const int LN = log_h + log_b;
-    const uint64_t total = (n << log_b) * width;
-    ScratchBuf tmp;
-    ZKB_TRY(tmp.alloc(total * sizeof(T), s));
-    ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F><<<grid_for(total, 256), 256, 0, s>>>(d_out, tmp.as<T>(), LN, width, total));
-    ZKB_CHECK_CUDA(cudaMemcpyAsync(d_out, tmp.p, total * sizeof(T), cudaMemcpyDeviceToDevice, s));
-  }
+  if (!bitrev) return bitrev_rows<F>(d_out, natural, log_h + log_b, width, s);
   return ZKB_OK;
 }
 
@@ -889,8 +902,7 @@ int ntt_dft_into(typename F::T *d, int log_h, uint32_t width, bool inverse, type
   T scale = 0;
   if (inverse) scale = Dom<F>::encode(inv_host<F>((T)(n % (uint64_t)F::P)));
   ZKB_TRY(run_passes<F>(d, tmp, log_h, width, 1, tw_buf, inverse, scale, s));
-  ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F><<<grid_for(n * width, 256), 256, 0, s>>>(tmp, d, log_h, width, n * width));
-  return ZKB_OK;
+  return bitrev_rows<F>(tmp, d, log_h, width, s);
 }
 
 template int ntt_dft_into<BabyBear>(uint32_t *, int, uint32_t, bool, uint32_t *, uint32_t *, cudaStream_t);

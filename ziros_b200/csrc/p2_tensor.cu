@@ -50,21 +50,41 @@ __device__ __forceinline__ void store8(uint32_t *out, const uint32_t (&o)[8]) {
   d[1] = make_uint4(o[4], o[5], o[6], o[7]);
 }
 
-// out += alpha-reduction of the chunk's columns (apow: one uint4 per column).
-__device__ __forceinline__ void combine8(uint64_t (&acc)[4], const uint32_t (&x)[8], const uint4 *__restrict__ apow,
+// acc += alpha-reduction of the chunk's columns (apow: one uint4 per column), times 2^32: four products to
+// a reduction (4 p^2 < 2^64; hi(t) - hi(m p) lies in (-p, 1.9 p)), the reduced sums in 64 bits.
+__device__ __forceinline__ void combine8(int64_t (&acc)[4], const uint32_t (&x)[8], const uint4 *__restrict__ apow,
                                          uint64_t c, uint64_t width) {
   using B = BabyBear;
 #pragma unroll
-  for (int i = 0; i < 8; i += 2) {
+  for (int i = 0; i < 8; i += 4) {
     if (c + i >= width) break;
-    const uint4 w0 = apow[c + i];
-    const uint4 w1 = c + i + 1 < width ? apow[c + i + 1] : make_uint4(0, 0, 0, 0);
-    acc[0] += B::mont_lazy_sum(x[i], w0.x, x[i + 1], w1.x);
-    acc[1] += B::mont_lazy_sum(x[i], w0.y, x[i + 1], w1.y);
-    acc[2] += B::mont_lazy_sum(x[i], w0.z, x[i + 1], w1.z);
-    acc[3] += B::mont_lazy_sum(x[i], w0.w, x[i + 1], w1.w);
+    uint64_t t[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint4 w = c + i + k < width ? apow[c + i + k] : make_uint4(0, 0, 0, 0);
+      t[0] += (uint64_t)x[i + k] * w.x;
+      t[1] += (uint64_t)x[i + k] * w.y;
+      t[2] += (uint64_t)x[i + k] * w.z;
+      t[3] += (uint64_t)x[i + k] * w.w;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t m = (uint32_t)t[k] * B::PINV;
+      acc[k] += (int64_t)(t[k] >> 32) - (int64_t)__umulhi(m, B::P);
+    }
   }
 }
+// The four sums; the multiple of p keeps a negative one positive (up to 2^32 columns' groups).
+__device__ __forceinline__ uint4 combined(const int64_t (&acc)[4]) {
+  constexpr int64_t BIAS = (int64_t)BabyBear::P << 31;
+  uint32_t r[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) r[k] = BabyBear::mont_reduce((uint64_t)(acc[k] + BIAS));
+  return make_uint4(r[0], r[1], r[2], r[3]);
+}
+
+// Brings a line of a later tile into L2 while this one computes.
+__device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // The tiles of 128 rows of a group: spread over the blocks first, so that the SMs' numbers of
 // tiles differ by one at most.
@@ -97,7 +117,7 @@ __global__ void __launch_bounds__(THREADS)
         for (int i = 0; i < 8; i++) x[i] = c + i < width ? fetch_col<BabyBear>(ml, row, c + i) : 0;
       }
     };
-    uint64_t acc[4] = {0, 0, 0, 0};
+    int64_t acc[4] = {0, 0, 0, 0};
     uint32_t x[8];
     load(x, 0);
 #pragma unroll 1
@@ -112,8 +132,7 @@ __global__ void __launch_bounds__(THREADS)
     if (live) {
       store8(digests + row * 8, o);
       if constexpr (COMBINE)
-        comb[row] = make_uint4(BabyBear::mont_reduce(acc[0]), BabyBear::mont_reduce(acc[1]), BabyBear::mont_reduce(acc[2]),
-                               BabyBear::mont_reduce(acc[3]));
+        comb[row] = combined(acc);
     }
   }
   teardown(sm, SPONGE);
@@ -148,7 +167,7 @@ __global__ void __launch_bounds__(THREADS)
       st8(g.tw + COL_Z, z);
       st8(g.tw + COL_Z + 8, z + 8);
     }
-    uint64_t acc[4] = {0, 0, 0, 0};
+    int64_t acc[4] = {0, 0, 0, 0};
     uint32_t x[8];
     load8(x, rp, 0, ncols, vec);
 #pragma unroll 1
@@ -173,7 +192,7 @@ __global__ void __launch_bounds__(THREADS)
     if constexpr (COMBINE) {
       if (live) {
         using B = BabyBear;
-        uint4 r = make_uint4(B::mont_reduce(acc[0]), B::mont_reduce(acc[1]), B::mont_reduce(acc[2]), B::mont_reduce(acc[3]));
+        uint4 r = combined(acc);
         if (!first) {
           const uint4 o = comb[row];
           r = make_uint4(B::add(o.x, r.x), B::add(o.y, r.y), B::add(o.z, r.z), B::add(o.w, r.w));
@@ -295,6 +314,8 @@ __global__ void __launch_bounds__(THREADS)
     const bool live = j < n_leaves;
     if (!live) j = n_leaves - 1;
     const uint4 *in = reinterpret_cast<const uint4 *>(e);
+    const uint64_t later = j + (uint64_t)gridDim.x * (blockDim.x / GROUP) * GROUP;
+    if (later < n_leaves) prefetch(in + (FOLD ? 4 : 2) * later);
     uint4 a, b;
     if constexpr (FOLD) {
       a = fold_ext4_one(in[4 * j], in[4 * j + 1], 2 * j, log_out, prm, itw);
