@@ -35,3 +35,21 @@ def test_dft_both_ways(oracle, field, width):
     f = d.dft_batch(t)
     assert (f == oracle.dft_batch(field, t)).all()
     assert (d.idft_batch(f) == t).all()
+
+
+@pytest.mark.parametrize("field,log_h,width", [(Z.GOLDILOCKS, 8, 1024), (Z.GOLDILOCKS, 12, 64), (Z.BABYBEAR, 12, 8)])
+@pytest.mark.parametrize("rev", [True, False])
+def test_trace_inside_the_output(field, log_h, width, rev):
+    """Two-pass plans read the trace before they write the output; heights of one 8-bit pass keep two."""
+    import torch
+    h = 1 << log_h
+    t = rand_field(field, (h, width), width)
+    d = Z.CudaDft(field)
+    want = d.coset_lde_batch(t, 1, bit_reverse_rows=rev)
+    for row0 in (0, h // 2, h):
+        out = torch.zeros((2 * h, width), dtype=torch.int32 if field == Z.BABYBEAR else torch.int64, device="cuda")
+        trace = out[row0:row0 + h]
+        trace.copy_(torch.from_numpy(t.view(np.int32 if field == Z.BABYBEAR else np.int64)))
+        d.coset_lde_batch_dev(trace, 1, out, bit_reverse_rows=rev)
+        torch.cuda.synchronize()
+        assert (out.cpu().numpy().view(t.dtype) == want).all()

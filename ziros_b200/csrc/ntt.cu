@@ -809,8 +809,13 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
     tn = *tune;
   }
   const uint64_t n = 1ull << log_h;
-  const int kmax = tn.kmax ? tn.kmax : plan_kmax<F>(d_trace, n, width, stride);
-  // Natural order: the transform goes to scratch, its rows then into the caller's buffer.
+  // A trace that lies in the output is read whole into scratch before the output is written, wherever a plan
+  // has two passes; so a one-pass plan of 8 bits is not taken for it.
+  const bool apart = (uintptr_t)(d_trace + n * stride) <= (uintptr_t)d_out ||
+                     (uintptr_t)(d_out + (n << log_b) * stride) <= (uintptr_t)d_trace;
+  const int kmax = tn.kmax ? tn.kmax : apart ? plan_kmax<F>(d_trace, n, width, stride) : pass_kmax<F>();
+  // Natural order: the transform goes to scratch, its rows then into the caller's buffer, which holds the
+  // coefficients until then (the fused kernel has read them all), so that one scratch buffer is enough.
   T *const natural = d_out;
   ScratchBuf reversed;
   if (!bitrev) {
@@ -832,6 +837,7 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
     const T *src = d_trace;
     if (ks.size() > 1) {
       T *cs = coef_scratch;
+      if (!cs && !bitrev && apart && ((uintptr_t)natural & 15) == 0) cs = natural;
       if (!cs) {
         ZKB_TRY(coef.alloc(n * width * sizeof(T), s));
         cs = coef.as<T>();
