@@ -598,7 +598,7 @@ def run_ours(args, wl: dict, rank: int, world: int, local_rank: int) -> int:
         hbm_peak, hbm_src = 6650.0, "of fallback"
     # NTT kernels: plain passes read and write their tiles once; the fused kernel reads the
     # coefficient matrix once and writes every coset block once
-    kmax = 10 if field == 0 else 7  # largest pass of the library's default plans
+    kmax = 10 if field == 0 else 8  # largest pass of the library's default plans at these sizes
     n_pass = -(-wl["log_h"] // kmax)
     b_blocks = 1 << lb
     ntt_roof = []
@@ -611,8 +611,9 @@ def run_ours(args, wl: dict, rank: int, world: int, local_rank: int) -> int:
             return None
         return (sum(g[0] for g in got), sum(g[1] for g in got), max(g[2] for g in got))
 
-    tile_loads = "tensor copy" if ("ntt_pass_tma" in kstats or "lde_fused_tma" in kstats) else "registers"
-    nk = kstat("ntt_pass", "ntt_pass_tma")
+    copied = ("ntt_pass_tma", "lde_fused_tma", "ntt_pass_tc", "lde_fused_tc")
+    tile_loads = "tensor copy" if any(k in kstats for k in copied) else "registers"
+    nk = kstat("ntt_pass", "ntt_pass_tma", "ntt_pass_tc")
     if nk and n_pass > 1:
         bytes_per_step = 2 * esize * (n * w * (n_pass - 1) + N_rows * w * (n_pass - 1))
         per_launch = bytes_per_step * args.steps / nk[0]
@@ -622,7 +623,7 @@ def run_ours(args, wl: dict, rank: int, world: int, local_rank: int) -> int:
                          "frac": ach / hbm_peak, "peak_source": hbm_src,
                          "algorithmic_bytes_per_launch": per_launch,
                          "traffic": traffic.get("ntt_pass") if traffic else None})
-    fk = kstat("lde_fused", "lde_fused_tma")
+    fk = kstat("lde_fused", "lde_fused_tma", "lde_fused_tc")
     if fk:
         per_launch = esize * (n * w + b_blocks * n * w)
         ach = per_launch / (fk[1] / fk[0] * 1e-3) / 1e9

@@ -186,7 +186,7 @@ ZKB_API int zkb_dft_batch_noalloc_dev(int field, void *d_rowmajor, uint32_t log_
  * Results are the same bit for bit.  No counterpart in the reference. */
 ZKB_API int zkb_set_ntt_tile_loads(int mode);
 /* Bounded device waits that gave up since the last call: tensor copies of the NTT tiles and
- * tensor-core products of the hashing kernels; nonzero means those outputs are
+ * tensor-core products of the NTT and hashing kernels; nonzero means those outputs are
  * invalid.  Resets the count. */
 ZKB_API int zkb_ntt_tile_load_errors(uint32_t *count);
 
