@@ -60,7 +60,7 @@ int permute_dev_impl(typename F::T *d_states, size_t n_elems, const typename F::
   ZKB_REQUIRE(rc != nullptr || n_rc == 0, "null round constants");
   const int field = sizeof(typename F::T) == 4 ? FIELD_BABYBEAR : FIELD_GOLDILOCKS;
   std::vector<uint64_t> rc64(rc, rc + n_rc);
-  std::vector<uint64_t> diag = p2_diagonal(field, 16);
+  const std::vector<uint64_t> &diag = p2_diagonal(field, 16);
   P2Params<F, 16> p;
   if (!build_p2_params<F, 16>(rc64.data(), n_rc, (int)n_ext, (int)n_int, diag.data(), 8, &p)) {
     set_error("round constants do not match n_external_rounds=%u n_internal_rounds=%u (n_rc=%zu)",

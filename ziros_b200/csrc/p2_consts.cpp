@@ -50,21 +50,29 @@ std::vector<uint64_t> p2_flat_constants(int field, int width, uint64_t seed) {
   return flat;
 }
 
-std::vector<uint64_t> p2_diagonal(int field, int width) {
-  if (field == FIELD_BABYBEAR && width == 16) {
-    // V = [-2, 1, 2, 1/2, 3, 4, -1/2, -3, -4, 1/2^8, 1/4, 1/8, 1/2^27, -1/2^8, -1/16, -1/2^27]
-    // (zkf-metal/src/poseidon2/babybear.rs:14-58)
-    const uint32_t P = BabyBear::P;
-    uint32_t inv2 = inv_host<BabyBear>(2);
-    auto ip = [&](int e) { return pow_host<BabyBear>(inv2, e); };
-    return {P - 2, 1, 2, inv2, 3, 4, P - inv2, P - 3, P - 4, ip(8), ip(2), ip(3), ip(27),
-            P - ip(8), P - ip(4), P - ip(27)};
-  }
-  if (field == FIELD_GOLDILOCKS && (width == 16 || width == 12)) {
-    const GoldilocksDiag g = goldilocks_diag(width);
-    return std::vector<uint64_t>(g.d, g.d + width);
-  }
-  return {};
+static std::vector<uint64_t> babybear_diagonal() {
+  // V = [-2, 1, 2, 1/2, 3, 4, -1/2, -3, -4, 1/2^8, 1/4, 1/8, 1/2^27, -1/2^8, -1/16, -1/2^27]
+  // (zkf-metal/src/poseidon2/babybear.rs:14-58)
+  const uint32_t P = BabyBear::P;
+  uint32_t inv2 = inv_host<BabyBear>(2);
+  auto ip = [&](int e) { return pow_host<BabyBear>(inv2, e); };
+  return {P - 2, 1, 2, inv2, 3, 4, P - inv2, P - 3, P - 4, ip(8), ip(2), ip(3), ip(27),
+          P - ip(8), P - ip(4), P - ip(27)};
+}
+
+static std::vector<uint64_t> goldilocks_diagonal(int width) {
+  const GoldilocksDiag g = goldilocks_diag(width);
+  return std::vector<uint64_t>(g.d, g.d + width);
+}
+
+// Made once: a batch permutation asks for it twice per call.
+const std::vector<uint64_t> &p2_diagonal(int field, int width) {
+  static const std::vector<uint64_t> bb16 = babybear_diagonal(), gl12 = goldilocks_diagonal(12),
+                                     gl16 = goldilocks_diagonal(16), none;
+  if (field == FIELD_BABYBEAR && width == 16) return bb16;
+  if (field == FIELD_GOLDILOCKS && width == 16) return gl16;
+  if (field == FIELD_GOLDILOCKS && width == 12) return gl12;
+  return none;
 }
 
 bool make_hasher_spec(int field, int width, uint64_t seed, HasherSpec *out) {

@@ -78,7 +78,7 @@ bool p2_round_numbers(int field, int width, int *rounds_f, int *rounds_p);
 std::vector<uint64_t> p2_flat_constants(int field, int width, uint64_t seed);
 // Canonical internal diagonal (BabyBear W16 V, Goldilocks W16 MATRIX_DIAG_16, the
 // self-generated Goldilocks W12 one).  Empty on unsupported configuration.
-std::vector<uint64_t> p2_diagonal(int field, int width);
+const std::vector<uint64_t> &p2_diagonal(int field, int width);
 
 // A fully described Poseidon2 hash configuration: permutation + sponge geometry
 // (PaddingFreeSponge<Perm, W, 8, OUT>, TruncatedPermutation<Perm, 2, OUT, W>).

@@ -402,7 +402,7 @@ static int prepare(K kernel, size_t smem) {
 // against 91), from there this one (32,768 x 8: 21.5 us against 24.7, x 64: 109 against 135).
 constexpr uint64_t MIN_ROWS = 148ull * GROUP + 1;
 
-bool takes(const P2Params<BabyBear, 16> &p, uint64_t rows) { return usable(p) && rows >= MIN_ROWS; }
+bool takes(const P2Params<BabyBear, 16> &p, uint64_t rows) { return rows >= MIN_ROWS && usable(p); }
 
 int hash_rows(const MatList &ml, uint64_t height, uint32_t *digests, const P2Params<BabyBear, 16> &p,
               const uint4 *apow, uint4 *comb, const char *name, cudaStream_t s) {

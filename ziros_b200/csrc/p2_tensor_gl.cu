@@ -277,7 +277,7 @@ constexpr uint64_t MIN_ROWS = 8192;
 
 template <int W>
 bool takes(const P2Params<Goldilocks, W> &p, uint64_t rows) {
-  return usable(p) && rows >= MIN_ROWS;
+  return rows >= MIN_ROWS && usable(p);
 }
 
 template <int W>

@@ -26,7 +26,7 @@ bool build_p2_params(const uint64_t *rc, size_t n_rc, int rounds_f, int rounds_p
   p->rate = 8;
   p->diag_kind = 0;
   {
-    const std::vector<uint64_t> v = p2_diagonal(sizeof(typename F::T) == 4 ? FIELD_BABYBEAR : FIELD_GOLDILOCKS, W);
+    const std::vector<uint64_t> &v = p2_diagonal(sizeof(typename F::T) == 4 ? FIELD_BABYBEAR : FIELD_GOLDILOCKS, W);
     bool same = true;
     for (int i = 0; i < W; i++) same = same && diag[i] == v[i];
     p->diag_kind = same ? 1 : 0;
