@@ -44,7 +44,7 @@
 namespace zkb {
 namespace {
 
-constexpr int MAX_BATCH = 1024;
+constexpr int MAX_BATCH = mt::MAX_JOBS;
 using mt::CompJob;
 using mt::LeafJob;
 

@@ -11,7 +11,18 @@ namespace zkb {
 namespace mt {
 struct LeafJob;
 struct CompJob;
+constexpr int MAX_JOBS = 1024;  // trees of one launch
 }  // namespace mt
+
+// The dynamic shared memory a kernel may be launched with.  The limit belongs to the function and the
+// context, not to the calling thread, and a smaller value lowers it for everyone: BYTES is one
+// constant per kernel, never the size of the launch at hand.
+template <int BYTES, class K>
+int smem_limit(K kernel) {
+  static_assert(BYTES <= 227 * 1024, "more shared memory than a block can have");
+  ZKB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES));
+  return ZKB_OK;
+}
 
 namespace p2t {
 

@@ -26,6 +26,10 @@ __device__ uint32_t g_p2t_wait_errors;
 namespace p2t {
 
 constexpr int THREADS = GROUP * MAX_GROUPS;
+// Shared memory of the many-tree kernels: the tables, then the jobs' starts.
+__host__ __device__ constexpr int mt_smem(Mode m, int jobs) {
+  return (smem_bytes(m) + 15) / 16 * 16 + jobs * (int)sizeof(uint64_t);
+}
 
 // Eight words of a row from column c on (zero past the end).
 __device__ __forceinline__ void load8(uint32_t (&x)[8], const uint32_t *rp, uint64_t c, uint64_t width, bool vec) {
@@ -248,7 +252,7 @@ __global__ void __launch_bounds__(THREADS)
     mt_leaf_kernel(const mt::LeafJob *__restrict__ jobs, int n_jobs, uint64_t tiles,
                    const __grid_constant__ P2Params<BabyBear, 16> p) {
   extern __shared__ __align__(128) uint8_t sm[];
-  uint64_t *starts = reinterpret_cast<uint64_t *>(sm + (smem_bytes(SPONGE_ANY) + 15) / 16 * 16);
+  uint64_t *starts = reinterpret_cast<uint64_t *>(sm + mt_smem(SPONGE_ANY, 0));
   for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].tile_start;
   Group g = setup(sm, p, SPONGE_ANY, 8, &g_p2t_wait_errors);
   P2T_TILES(t, tiles) {
@@ -280,7 +284,7 @@ __global__ void __launch_bounds__(THREADS)
     mt_compress_kernel(const mt::CompJob *__restrict__ jobs, int n_jobs, uint64_t total,
                        const __grid_constant__ P2Params<BabyBear, 16> p) {
   extern __shared__ __align__(128) uint8_t sm[];
-  uint64_t *starts = reinterpret_cast<uint64_t *>(sm + (smem_bytes(STATE16) + 15) / 16 * 16);
+  uint64_t *starts = reinterpret_cast<uint64_t *>(sm + mt_smem(STATE16, 0));
   for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].start;
   Group g = setup(sm, p, STATE16, 8, &g_p2t_wait_errors);
   const uint64_t tiles = (total + GROUP - 1) / GROUP;
@@ -390,13 +394,6 @@ static Shape shape(uint64_t tiles, uint64_t perms, int sms) {
   return {(unsigned)std::min<uint64_t>(sms, tiles), (unsigned)(best * GROUP)};
 }
 
-template <class K>
-static int prepare(K kernel, size_t smem) {
-  // sticky per kernel and context; cheap
-  ZKB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  return ZKB_OK;
-}
-
 // Smallest number of rows (or compressions) in one launch: more than one tile an SM.  Up to there
 // the quad form is the faster one (16,384 rows x 32 columns: 46 us against 55; 18,944 x 64: 86
 // against 91), from there this one (32,768 x 8: 21.5 us against 24.7, x 64: 109 against 135).
@@ -413,10 +410,10 @@ int hash_rows(const MatList &ml, uint64_t height, uint32_t *digests, const P2Par
   const size_t smem = smem_bytes(SPONGE);
   const bool vec = ml.n == 1 && width % 4 == 0 && ((uintptr_t)ml.ptr[0] & 15) == 0;
   if (comb) {
-    ZKB_TRY(prepare(leaf_kernel<true>, smem));
+    ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(leaf_kernel<true>));
     ZKB_LAUNCH(name, s, leaf_kernel<true><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, apow, comb, vec));
   } else {
-    ZKB_TRY(prepare(leaf_kernel<false>, smem));
+    ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(leaf_kernel<false>));
     ZKB_LAUNCH(name, s, leaf_kernel<false><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, apow, comb, vec));
   }
   return ZKB_OK;
@@ -431,10 +428,10 @@ int hash_slab(const uint32_t *mat, uint64_t stride, uint64_t c0, uint64_t ncols,
   const size_t smem = smem_bytes(SPONGE);
   const bool vec = stride % 4 == 0 && c0 % 4 == 0 && ncols % 4 == 0 && ((uintptr_t)mat & 15) == 0;
   if (apow) {
-    ZKB_TRY(prepare(slab_kernel<true>, smem));
+    ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(slab_kernel<true>));
     ZKB_LAUNCH(name, s, slab_kernel<true><<<sh.grid, sh.threads, smem, s>>>(mat, stride, c0, ncols, height, carry, first, last, digests, p, apow, comb, vec));
   } else {
-    ZKB_TRY(prepare(slab_kernel<false>, smem));
+    ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(slab_kernel<false>));
     ZKB_LAUNCH(name, s, slab_kernel<false><<<sh.grid, sh.threads, smem, s>>>(mat, stride, c0, ncols, height, carry, first, last, digests, p, apow, comb, vec));
   }
   return ZKB_OK;
@@ -446,7 +443,7 @@ int compress(const uint32_t *prev, uint32_t *next, uint64_t n_out, const uint32_
   ZKB_TRY(current_context(&ctx));
   const Shape sh = shape((n_out + GROUP - 1) / GROUP, 1, ctx->sm_count);
   const size_t smem = smem_bytes(STATE16);
-  ZKB_TRY(prepare(compress_kernel, smem));
+  ZKB_TRY(smem_limit<smem_bytes(STATE16)>(compress_kernel));
   ZKB_LAUNCH(name, s, compress_kernel<<<sh.grid, sh.threads, smem, s>>>(prev, next, n_out, inj, inj_h, p));
   return ZKB_OK;
 }
@@ -456,8 +453,9 @@ int mt_leaf(const mt::LeafJob *d_jobs, int n, uint64_t tiles, uint64_t perms, co
   DeviceContext *ctx;
   ZKB_TRY(current_context(&ctx));
   const Shape sh = shape(tiles, perms, ctx->sm_count);
-  const size_t smem = (smem_bytes(SPONGE_ANY) + 15) / 16 * 16 + n * sizeof(uint64_t);
-  ZKB_TRY(prepare(mt_leaf_kernel, smem));
+  ZKB_REQUIRE(n <= mt::MAX_JOBS, "internal: %d trees in one launch", n);
+  const size_t smem = mt_smem(SPONGE_ANY, n);
+  ZKB_TRY(smem_limit<mt_smem(SPONGE_ANY, mt::MAX_JOBS)>(mt_leaf_kernel));
   ZKB_LAUNCH(name, s, mt_leaf_kernel<<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, tiles, p));
   return ZKB_OK;
 }
@@ -467,8 +465,9 @@ int mt_compress(const mt::CompJob *d_jobs, int n, uint64_t total, const P2Params
   DeviceContext *ctx;
   ZKB_TRY(current_context(&ctx));
   const Shape sh = shape((total + GROUP - 1) / GROUP, 1, ctx->sm_count);
-  const size_t smem = (smem_bytes(STATE16) + 15) / 16 * 16 + n * sizeof(uint64_t);
-  ZKB_TRY(prepare(mt_compress_kernel, smem));
+  ZKB_REQUIRE(n <= mt::MAX_JOBS, "internal: %d trees in one launch", n);
+  const size_t smem = mt_smem(STATE16, n);
+  ZKB_TRY(smem_limit<mt_smem(STATE16, mt::MAX_JOBS)>(mt_compress_kernel));
   ZKB_LAUNCH(name, s, mt_compress_kernel<<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, total, p));
   return ZKB_OK;
 }
@@ -481,10 +480,10 @@ int fri_fold_hash(const uint32_t *e, uint32_t *out, uint64_t n_leaves, int log_o
   const Shape sh = shape((n_leaves + GROUP - 1) / GROUP, 1, ctx->sm_count);
   const size_t smem = smem_bytes(SPONGE);
   if (prm) {
-    ZKB_TRY(prepare(fri_kernel<true>, smem));
+    ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(fri_kernel<true>));
     ZKB_LAUNCH(name, s, fri_kernel<true><<<sh.grid, sh.threads, smem, s>>>(e, out, n_leaves, log_out, *prm, itw, digests, p));
   } else {
-    ZKB_TRY(prepare(fri_kernel<false>, smem));
+    ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(fri_kernel<false>));
     ZKB_LAUNCH(name, s, fri_kernel<false><<<sh.grid, sh.threads, smem, s>>>(e, out, n_leaves, log_out, Ext4Params{}, itw, digests, p));
   }
   return ZKB_OK;
@@ -495,7 +494,7 @@ int permute(uint32_t *states, uint64_t n, const P2Params<BabyBear, 16> &p, cudaS
   ZKB_TRY(current_context(&ctx));
   const Shape sh = shape((n + GROUP - 1) / GROUP, 1, ctx->sm_count);
   const size_t smem = smem_bytes(PERM16);
-  ZKB_TRY(prepare(permute_kernel, smem));
+  ZKB_TRY(smem_limit<smem_bytes(PERM16)>(permute_kernel));
   const bool vec = ((uintptr_t)states & 15) == 0;
   ZKB_LAUNCH("p2_permute", s, permute_kernel<<<sh.grid, sh.threads, smem, s>>>(states, n, vec, p));
   return ZKB_OK;

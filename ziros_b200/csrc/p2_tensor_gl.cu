@@ -24,6 +24,12 @@ constexpr int out_words() {
   return W == 16 ? 8 : 4;
 }
 
+// Shared memory of the many-tree kernels: the tables, then the jobs' starts.
+template <int W>
+__host__ __device__ constexpr int mt_smem(int jobs) {
+  return (Shape<W>::SMEM + 15) / 16 * 16 + jobs * (int)sizeof(uint64_t);
+}
+
 // Eight words of a row from column c on (zero past the end).
 __device__ __forceinline__ void load8(uint64_t (&x)[8], const uint64_t *rp, uint64_t c, uint64_t width, bool vec) {
   if (vec && c + 8 <= width) {
@@ -121,7 +127,7 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     mt_leaf_kernel(const mt::LeafJob *__restrict__ jobs, int n_jobs, uint64_t tiles,
                    const __grid_constant__ P2Params<Goldilocks, W> p) {
   extern __shared__ __align__(128) uint8_t sm[];
-  uint64_t *starts = reinterpret_cast<uint64_t *>(sm + (Shape<W>::SMEM + 15) / 16 * 16);
+  uint64_t *starts = reinterpret_cast<uint64_t *>(sm + mt_smem<W>(0));
   for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].tile_start;
   Group g = setup<W>(sm, p, true, &g_p2g_wait_errors);
   P2G_TILES(t, tiles) {
@@ -191,7 +197,7 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
                        const __grid_constant__ P2Params<Goldilocks, W> p) {
   extern __shared__ __align__(128) uint8_t sm[];
   constexpr int OUT = out_words<W>();
-  uint64_t *starts = reinterpret_cast<uint64_t *>(sm + (Shape<W>::SMEM + 15) / 16 * 16);
+  uint64_t *starts = reinterpret_cast<uint64_t *>(sm + mt_smem<W>(0));
   for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].start;
   Group g = setup<W>(sm, p, false, &g_p2g_wait_errors);
   const uint64_t tiles = (total + GROUP - 1) / GROUP;
@@ -264,12 +270,6 @@ static Launch shape(uint64_t tiles, uint64_t perms, int sms) {
   return {(unsigned)std::min<uint64_t>(sms, tiles), (unsigned)(best * GROUP)};
 }
 
-template <class K>
-static int prepare(K kernel, size_t smem) {
-  ZKB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  return ZKB_OK;
-}
-
 // Smallest number of rows (or compressions) in one launch; against quads of threads (p2_quad.cuh),
 // width 12 and 16: 4,096 rows x 32 columns 94 us and 113 against 84 and 81, 8,192 100 and 114 against
 // 126 and 120, 16,384 98 and 116 against 224 and 216.
@@ -288,7 +288,7 @@ int hash_rows(const MatList &ml, uint64_t height, uint64_t *digests, const P2Par
   const Launch sh = shape<W>((height + GROUP - 1) / GROUP, (ml.col_start[ml.n] + 7) / 8, ctx->sm_count);
   const size_t smem = Shape<W>::SMEM;
   const bool vec = ml.n == 1 && ml.width[0] % 2 == 0 && ((uintptr_t)ml.ptr[0] & 15) == 0;
-  ZKB_TRY(prepare(leaf_kernel<W>, smem));
+  ZKB_TRY(smem_limit<Shape<W>::SMEM>(leaf_kernel<W>));
   ZKB_LAUNCH(name, s, leaf_kernel<W><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, vec));
   return ZKB_OK;
 }
@@ -300,7 +300,7 @@ int compress(const uint64_t *prev, uint64_t *next, uint64_t n_out, const uint64_
   ZKB_TRY(current_context(&ctx));
   const Launch sh = shape<W>((n_out + GROUP - 1) / GROUP, 1, ctx->sm_count);
   const size_t smem = Shape<W>::SMEM;
-  ZKB_TRY(prepare(compress_kernel<W>, smem));
+  ZKB_TRY(smem_limit<Shape<W>::SMEM>(compress_kernel<W>));
   ZKB_LAUNCH(name, s, compress_kernel<W><<<sh.grid, sh.threads, smem, s>>>(prev, next, n_out, inj, inj_h, p));
   return ZKB_OK;
 }
@@ -311,8 +311,9 @@ int mt_leaf(const mt::LeafJob *d_jobs, int n, uint64_t tiles, uint64_t perms, co
   DeviceContext *ctx;
   ZKB_TRY(current_context(&ctx));
   const Launch sh = shape<W>(tiles, perms, ctx->sm_count);
-  const size_t smem = (Shape<W>::SMEM + 15) / 16 * 16 + n * sizeof(uint64_t);
-  ZKB_TRY(prepare(mt_leaf_kernel<W>, smem));
+  ZKB_REQUIRE(n <= mt::MAX_JOBS, "internal: %d trees in one launch", n);
+  const size_t smem = mt_smem<W>(n);
+  ZKB_TRY(smem_limit<mt_smem<W>(mt::MAX_JOBS)>(mt_leaf_kernel<W>));
   ZKB_LAUNCH(name, s, mt_leaf_kernel<W><<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, tiles, p));
   return ZKB_OK;
 }
@@ -323,8 +324,9 @@ int mt_compress(const mt::CompJob *d_jobs, int n, uint64_t total, const P2Params
   DeviceContext *ctx;
   ZKB_TRY(current_context(&ctx));
   const Launch sh = shape<W>((total + GROUP - 1) / GROUP, 1, ctx->sm_count);
-  const size_t smem = (Shape<W>::SMEM + 15) / 16 * 16 + n * sizeof(uint64_t);
-  ZKB_TRY(prepare(mt_compress_kernel<W>, smem));
+  ZKB_REQUIRE(n <= mt::MAX_JOBS, "internal: %d trees in one launch", n);
+  const size_t smem = mt_smem<W>(n);
+  ZKB_TRY(smem_limit<mt_smem<W>(mt::MAX_JOBS)>(mt_compress_kernel<W>));
   ZKB_LAUNCH(name, s, mt_compress_kernel<W><<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, total, p));
   return ZKB_OK;
 }
@@ -335,7 +337,7 @@ int permute(uint64_t *states, uint64_t n, const P2Params<Goldilocks, W> &p, cuda
   ZKB_TRY(current_context(&ctx));
   const Launch sh = shape<W>((n + GROUP - 1) / GROUP, 1, ctx->sm_count);
   const size_t smem = Shape<W>::SMEM;
-  ZKB_TRY(prepare(permute_kernel<W>, smem));
+  ZKB_TRY(smem_limit<Shape<W>::SMEM>(permute_kernel<W>));
   ZKB_LAUNCH("p2_permute", s, permute_kernel<W><<<sh.grid, sh.threads, smem, s>>>(states, n, p));
   return ZKB_OK;
 }
