@@ -67,6 +67,9 @@ ZKB_API int zkb_set_device(int device);
  * on device work has a deadline (env ZKB_WATCHDOG_MS, default 120000; 0 = none).  A
  * device error or an expired deadline opens a process-wide circuit; while it is open,
  * every compute entry point declines (ZKB_DECLINED: the caller takes its CPU path).
+ * Waits inside the kernels (for tensor copies and tensor-core products) are bounded too:
+ * when one has given up, the next call that waits for the device fails with
+ * ZKB_ERR_TIMEOUT instead of returning a wrong root, and opens the circuit.
  * ZKB_DISABLE=1 declines everything (kill switch, like the reference's ZKF_METAL). */
 ZKB_API int zkb_circuit_open(char *why_out, size_t cap);  /* 1 open (reason copied), 0 closed */
 ZKB_API void zkb_circuit_reset(void);
@@ -86,6 +89,9 @@ ZKB_API int zkb_get_thresholds(zkb_thresholds *thresholds_out);
  * next `count` device allocations fail as out of memory; kind 2: the next `count` stream
  * waits report an expired deadline (after the work has finished). */
 ZKB_API int zkb_debug_inject_fault(int kind, int count);
+/* For tests: one block whose wait for a tensor-core product that nothing issues gives up after
+ * `polls` (1..4096) polls.  No counterpart in the reference. */
+ZKB_API int zkb_debug_wait_expiry(uint32_t polls, void *stream);
 /* Number of device allocations (stream-ordered pool or cudaMalloc) the library has
  * made in this process.  Tests read it around a call to check that the call allocated
  * nothing.  No counterpart in the reference. */
@@ -187,7 +193,8 @@ ZKB_API int zkb_dft_batch_noalloc_dev(int field, void *d_rowmajor, uint32_t log_
 ZKB_API int zkb_set_ntt_tile_loads(int mode);
 /* Bounded device waits that gave up since the last call: tensor copies of the NTT tiles and
  * tensor-core products of the NTT and hashing kernels; nonzero means those outputs are
- * invalid.  Resets the count. */
+ * invalid.  Resets the count.  (Calls that wait for the device report it by themselves, see
+ * failure detection; this one is for outputs of asynchronous calls.) */
 ZKB_API int zkb_ntt_tile_load_errors(uint32_t *count);
 
 /* p3 coset_lde_batch(trace, log_blowup, shift) followed, when bitrev_rows=1, by

@@ -186,6 +186,7 @@ SIGNATURES = {
     "zkb_circuit_open": (_I, [C.c_char_p, _SZ]),
     "zkb_circuit_reset": (None, []),
     "zkb_debug_inject_fault": (_I, [_I, _I]),
+    "zkb_debug_wait_expiry": (_I, [_U32, _P]),
     "zkb_batch_set_merkle_fusion": (_I, [_P, _U32, _U32]),
     "zkb_batch_queue_info": (_I, [_P, _P]),
     "zkb_batch_profile": (_I, [_P, _P, _P, _P]),
@@ -266,6 +267,11 @@ def inject_fault(kind: int, count: int = 1) -> None:
     check(load().zkb_debug_inject_fault(kind, count))
 
 
+def debug_wait_expiry(polls: int, stream=None) -> None:
+    """For tests: a kernel whose bounded wait gives up after `polls` polls."""
+    check(load().zkb_debug_wait_expiry(polls, stream))
+
+
 def device_allocations() -> int:
     """Device allocations the library has made in this process (pool or cudaMalloc)."""
     return int(load().zkb_debug_device_allocations())
@@ -287,7 +293,7 @@ def set_ntt_tile_loads(mode: int) -> None:
 
 
 def ntt_tile_load_errors() -> int:
-    """Tensor-copy waits of the NTT passes that gave up since the last call (resets)."""
+    """Bounded waits inside kernels that gave up since the last call (resets)."""
     n = C.c_uint32(0)
     check(load().zkb_ntt_tile_load_errors(C.byref(n)))
     return n.value

@@ -10,12 +10,11 @@
 
 #include "common.cuh"
 #include "engine.cuh"
-#include "ntt_tc.cuh"
-#include "p2_launch.cuh"
 
 namespace zkb {
 const char *last_error();
 int measure_mul_peak(int field, double *mul_per_s);
+int debug_wait_expiry(uint32_t polls, cudaStream_t s);
 }
 
 using namespace zkb;
@@ -167,6 +166,12 @@ int zkb_debug_inject_fault(int kind, int count) {
   return rc;
 }
 
+int zkb_debug_wait_expiry(uint32_t polls, void *stream) {
+  ZKB_ENTRY();
+  ZKB_REQUIRE(polls >= 1 && polls <= 4096, "poll limit %u (1..4096)", polls);
+  return debug_wait_expiry(polls, resolve_stream(stream));
+}
+
 uint64_t zkb_debug_device_allocations(void) { return device_alloc_count(); }
 uint64_t zkb_debug_pool_allocations(void) { return pool_alloc_count(); }
 
@@ -276,13 +281,7 @@ int zkb_set_ntt_tile_loads(int mode) {
 int zkb_ntt_tile_load_errors(uint32_t *count) {
   ZKB_ENTRY();
   ZKB_REQUIRE(count != nullptr, "null count");
-  uint32_t bb = 0, gl = 0, tc = 0;
-  ZKB_TRY(ntt_tc::wait_errors(&tc));
-  ZKB_TRY(p2t::wait_errors(&bb));
-  ZKB_TRY(p2g::wait_errors(&gl));
-  ZKB_TRY(ntt_tma_wait_errors(count));
-  *count += bb + gl + tc;
-  return ZKB_OK;
+  return take_wait_errors(count);
 }
 
 int zkb_dft_batch(int field, void *rowmajor, uint32_t log_h, uint32_t width, int inverse) {

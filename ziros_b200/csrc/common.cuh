@@ -58,6 +58,7 @@ struct DeviceTable {
 struct DeviceContext {
   int device = -1;
   int sm_count = 0;
+  uint32_t *wait_word = nullptr;  // where kernels count bounded waits that gave up (see report_wait)
   std::mutex mu;
   std::map<std::tuple<int, int, int>, DeviceTable> twiddles;           // (field, log_n, inverse)
   std::map<std::tuple<int, int, int, uint64_t>, DeviceTable> cosets;   // (field, log_n, log_b, shift)
@@ -67,6 +68,18 @@ struct DeviceContext {
 
 // Context of the calling thread's current device (initialised on first use).
 int current_context(DeviceContext **out);
+// Bounded device waits that gave up.  Kernels count them in one word of page-locked host memory (every
+// device's address of it is DeviceContext::wait_word), so that the host sees them after any wait for a
+// stream at no cost to the calls in which nothing gives up.  While the word has moved since it was last
+// acknowledged (circuit_reset, take_wait_errors), wait_stream fails: what kernels produced since then is
+// not to be used.
+int take_wait_errors(uint32_t *count);  // since the last call; acknowledges them
+#ifdef __CUDACC__
+__device__ __forceinline__ void report_wait(uint32_t *word) {
+  atomicAdd(word, 1u);
+  __threadfence_system();
+}
+#endif
 // Stream of the calling thread on its current device (created on first use).
 cudaStream_t thread_stream();
 // A user stream argument follows CUDA's convention: NULL is the default stream.
@@ -85,7 +98,7 @@ uint64_t pool_alloc_count();
 // memory back to the device (for allocations outside the pool, e.g. a batch plan's arena).
 int release_cached_memory();
 // Host wait on a stream with the watchdog deadline (ZKB_WATCHDOG_MS, default 120 s, 0 =
-// none); a device error or an expired deadline opens the circuit.
+// none); a device error, an expired deadline or a device wait that gave up opens the circuit.
 int wait_stream(cudaStream_t s);
 bool library_disabled();
 // ZKB_DECLINED (with the reason) when the library is disabled or the circuit is open.

@@ -35,6 +35,29 @@ const char *last_error() { return g_last_error.c_str(); }
 static std::mutex g_ctx_mu;
 static std::vector<std::unique_ptr<DeviceContext>> g_ctx;
 
+// ---- waits that gave up: a page of this library's own memory, registered with the driver
+namespace {
+alignas(4096) volatile uint32_t g_wait_page[1024];  // [0] counts
+std::atomic<uint32_t> g_wait_reported{0}, g_wait_acknowledged{0};
+
+int wait_word(uint32_t **dev) {
+  // the first call of a process may come under stream capture, where registering is allowed in the
+  // relaxed mode only
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  ZKB_CHECK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  void *page = const_cast<uint32_t *>(g_wait_page);
+  cudaError_t e = cudaHostRegister(page, sizeof g_wait_page, cudaHostRegisterPortable | cudaHostRegisterMapped);
+  if (e == cudaErrorHostMemoryAlreadyRegistered) {
+    cudaGetLastError();
+    e = cudaSuccess;
+  }
+  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)dev, page, 0);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  ZKB_CHECK_CUDA(e);
+  return ZKB_OK;
+}
+}  // namespace
+
 int current_context(DeviceContext **out) {
   int dev = 0;
   ZKB_CHECK_CUDA(cudaGetDevice(&dev));
@@ -44,6 +67,7 @@ int current_context(DeviceContext **out) {
     auto c = std::make_unique<DeviceContext>();
     c->device = dev;
     ZKB_CHECK_CUDA(cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, dev));
+    ZKB_TRY(wait_word(&c->wait_word));
     // Keep freed scratch in the pool: commits of the same shape reuse it without
     // returning memory to the driver between calls.  A block freed on one stream is reused
     // on another only once its free has completed (or the stream already waits for it):
@@ -257,6 +281,21 @@ void circuit_reset() {
   std::lock_guard<std::mutex> lk(g_circuit_mu);
   g_circuit.store(false);
   g_circuit_why.clear();
+  g_wait_acknowledged.store(g_wait_page[0]);
+}
+
+int take_wait_errors(uint32_t *count) {
+  // an event of the default stream: what streams that synchronise with it have done is counted
+  cudaEvent_t e;
+  ZKB_CHECK_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  cudaError_t err = cudaEventRecord(e, nullptr);
+  if (err == cudaSuccess) err = cudaEventSynchronize(e);
+  cudaEventDestroy(e);
+  ZKB_CHECK_CUDA(err);
+  const uint32_t now = g_wait_page[0];
+  *count = now - g_wait_reported.exchange(now);
+  g_wait_acknowledged.store(now);
+  return ZKB_OK;
 }
 
 int inject_fault(int kind, int count) {
@@ -305,6 +344,11 @@ int wait_stream(cudaStream_t s) {
     trip_circuit(cudaGetErrorString(e));
     set_error("device work failed: %s", cudaGetErrorString(e));
     return ZKB_ERR_CUDA;
+  }
+  if (g_wait_page[0] != g_wait_acknowledged.load()) {
+    trip_circuit("a bounded wait inside a kernel gave up");
+    set_error("a bounded wait inside a kernel gave up: the results are invalid");
+    return ZKB_ERR_TIMEOUT;
   }
   return ZKB_OK;
 }

@@ -7,6 +7,7 @@
 // multiply throughput it sustains once its additions and data movement are paid.
 #include "common.cuh"
 #include "field.cuh"
+#include "tcgen05.cuh"
 
 namespace zkb {
 
@@ -59,6 +60,31 @@ static int mul_peak(double *mul_per_s) {
 int measure_mul_peak(int field, double *mul_per_s) {
   if (field == ZKB_FIELD_BABYBEAR) return mul_peak<BabyBear>(mul_per_s);
   return mul_peak<Goldilocks>(mul_per_s);
+}
+
+// A group of the hashing kernels waits for a product that nothing issued, `polls` polls long (about 4 us
+// each), then goes on to a second layer and ends.
+__global__ void __launch_bounds__(128) wait_expiry_kernel(uint32_t polls, uint32_t *waits) {
+  __shared__ __align__(16) uint8_t sm[16];
+  const uint32_t mbar = (uint32_t)__cvta_generic_to_shared(sm) + 8;
+  if (threadIdx.x == 0) {
+    *reinterpret_cast<uint32_t *>(sm) = 0;
+    tc::init_barrier(mbar);
+    tc::init_fence();
+  }
+  __syncthreads();
+  tc::Group g = tc::make_group(sm, 0, mbar, 0, waits);
+  g.one = 0;
+  g.polls = polls;
+  tc::finish(g);
+  tc::finish(g);
+}
+
+int debug_wait_expiry(uint32_t polls, cudaStream_t s) {
+  DeviceContext *ctx;
+  ZKB_TRY(current_context(&ctx));
+  ZKB_LAUNCH("debug_wait_expiry", s, wait_expiry_kernel<<<1, 128, 0, s>>>(polls, ctx->wait_word));
+  return ZKB_OK;
 }
 
 }  // namespace zkb

@@ -146,10 +146,9 @@ struct FriProof {
 };
 
 // Tile loads of the NTT passes (0 = coalesced loads into registers, 1 = one tensor copy
-// per tile), and the count of tensor-copy waits that gave up (reset on read).
+// per tile).
 void set_ntt_tile_loads(int mode);
 int ntt_tile_loads_mode();
-int ntt_tma_wait_errors(uint32_t *count);
 
 // The PCIe link of an engine, handed out one trace piece at a time.  Among the waiting
 // uploads the one with the fewest bytes left goes next (ties: the earlier ticket, taken

@@ -273,13 +273,11 @@ constexpr size_t tma_bar_off() {
   return (pass_tile_smem<F, LR1, LR2, C>() + 15) & ~(size_t)15;
 }
 
-__device__ uint32_t g_tma_wait_errors;
-
 template <class F, int LR1, int LR2, int C>
 __global__ void __launch_bounds__(C << LR2)
     ntt_pass_tma_kernel(const typename F::T *in, typename F::T *out, const PassGeom g,
                         const typename F::T *__restrict__ tw, typename F::T post_scale,
-                        const __grid_constant__ SmallTw<F> st, const __grid_constant__ CUtensorMap map) {
+                        const __grid_constant__ SmallTw<F> st, const __grid_constant__ CUtensorMap map, uint32_t *waits) {
   extern __shared__ __align__(128) unsigned char tma_smem[];  // the tensor copy's destination
   constexpr int K = LR1 + LR2;
   uint64_t *bar = reinterpret_cast<uint64_t *>(tma_smem + tma_bar_off<F, LR1, LR2, C>());
@@ -294,7 +292,7 @@ __global__ void __launch_bounds__(C << LR2)
   }
   __syncthreads();  // the barrier is initialised before anyone waits on it
   ntt_pass_tile<F, LR1, LR2, C, false, true>(in, out, g, tw, post_scale, st, blockIdx.x, tma_smem, bar,
-                                             &g_tma_wait_errors);
+                                             waits);
 }
 
 // Tile loads of the passes and the fused middle: 1 = one tensor copy per tile (the
@@ -367,11 +365,13 @@ static int launch_pass_tma_c(const typename F::T *src, typename F::T *out, const
                              const SmallTw<F> &st, cudaStream_t s) {
   constexpr unsigned threads = C << LR2;
   const size_t smem = tma_bar_off<F, LR1, LR2, C>() + 16;
+  DeviceContext *ctx;
+  ZKB_TRY(current_context(&ctx));
   CUtensorMap map;
   ZKB_TRY(pass_tensor_map(&map, src, sizeof(typename F::T), g, cols, LR1 + LR2, n_blocks, C));
   ZKB_CHECK_CUDA(cudaFuncSetAttribute(ntt_pass_tma_kernel<F, LR1, LR2, C>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  ZKB_LAUNCH("ntt_pass_tma", s, ntt_pass_tma_kernel<F, LR1, LR2, C><<<(unsigned)ctas, threads, smem, s>>>(src, out, g, tw, scale, st, map));
+  ZKB_LAUNCH("ntt_pass_tma", s, ntt_pass_tma_kernel<F, LR1, LR2, C><<<(unsigned)ctas, threads, smem, s>>>(src, out, g, tw, scale, st, map, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(C << LR2)
                          const typename F::T *__restrict__ itw, const typename F::T *__restrict__ ftw,
                          const typename F::T *__restrict__ ctab_t, const typename F::T *__restrict__ ftw_t,
                          const __grid_constant__ SmallTw<F> ist, const __grid_constant__ SmallTw<F> fst,
-                         const __grid_constant__ CUtensorMap map) {
+                         const __grid_constant__ CUtensorMap map, uint32_t *waits) {
   extern __shared__ __align__(128) unsigned char tma_smem[];
   constexpr int K = LR1 + LR2;
   uint64_t *bar = reinterpret_cast<uint64_t *>(tma_smem + fused_bar_off<F, LR1, LR2, C>());
@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(C << LR2)
   }
   __syncthreads();  // the barrier is initialised before anyone waits on it
   lde_fused_tile<F, LR1, LR2, C, false, true>(in, out, g, itw, ftw, ctab_t, ftw_t, ist, fst, blockIdx.x, tma_smem,
-                                              bar, &g_tma_wait_errors);
+                                              bar, waits);
 }
 
 template <class F, int LR1, int LR2, int C>
@@ -646,10 +646,12 @@ static int launch_fused_c(const typename F::T *in, typename F::T *out, const Fus
     CUtensorMap map;
     ZKB_TRY(pass_tensor_map(&map, in, sizeof(T), pg, cols, LR1 + LR2, 1, C));
     const size_t smem = fused_bar_off<F, LR1, LR2, C>() + 16;
+    DeviceContext *ctx;
+    ZKB_TRY(current_context(&ctx));
     ZKB_CHECK_CUDA(cudaFuncSetAttribute(lde_fused_tma_kernel<F, LR1, LR2, C>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     const SmallTw<F> ist = small_twiddles<F>(true), fst = small_twiddles<F>(false);
-    ZKB_LAUNCH("lde_fused_tma", s, lde_fused_tma_kernel<F, LR1, LR2, C><<<(unsigned)ctas0, threads, smem, s>>>(in, out, g, itw, ftw, ctab, ftw_t, ist, fst, map));
+    ZKB_LAUNCH("lde_fused_tma", s, lde_fused_tma_kernel<F, LR1, LR2, C><<<(unsigned)ctas0, threads, smem, s>>>(in, out, g, itw, ftw, ctab, ftw_t, ist, fst, map, ctx->wait_word));
     return ZKB_OK;
   }
   const size_t smem = fused_tile_smem<F, LR1, LR2, C>();
@@ -938,14 +940,5 @@ template int ntt_lde_dev<Goldilocks>(const uint64_t *, int, uint32_t, int, uint6
 
 void set_ntt_tile_loads(int mode) { ntt_tile_loads().store(mode); }
 int ntt_tile_loads_mode() { return ntt_tile_loads().load(); }
-
-int ntt_tma_wait_errors(uint32_t *count) {
-  uint32_t v = 0;
-  ZKB_CHECK_CUDA(cudaMemcpyFromSymbol(&v, g_tma_wait_errors, sizeof v));
-  const uint32_t zero = 0;
-  ZKB_CHECK_CUDA(cudaMemcpyToSymbol(g_tma_wait_errors, &zero, sizeof zero));
-  *count = v;
-  return ZKB_OK;
-}
 
 }  // namespace zkb

@@ -24,8 +24,6 @@
 
 namespace zkb {
 
-__device__ uint32_t g_ntt_tc_wait_errors;
-
 namespace ntt_tc {
 using namespace tc;
 
@@ -118,7 +116,7 @@ __device__ __forceinline__ void tile_copy(const T *tile, const CUtensorMap *map,
 }
 __device__ __forceinline__ void group_wait(Group &g, uint32_t mbar, uint32_t &phase) {
   if (!wait_parity(mbar, phase, g.polls)) {
-    if (g.polls) atomicAdd(g.err, 1u);
+    if (g.polls) report_wait(g.err);
     g.polls = 0;
   }
   phase ^= 1;
@@ -165,7 +163,7 @@ __device__ __forceinline__ void dft(Group &g, int matrix, Get get, Put put, Afte
 template <int LA, int LB, int C>
 __global__ void __launch_bounds__(ROWS * Tile<LA, LB, C>::GROUPS, 1)
     pass_kernel(T *out, const PassGeom g, uint64_t tiles, const T *__restrict__ tw, int inverse, T post_scale,
-                const __grid_constant__ CUtensorMap map) {
+                const __grid_constant__ CUtensorMap map, uint32_t *waits) {
   using S = Tile<LA, LB, C>;
   constexpr int K = S::K, RA = S::RA, RB = S::RB;
   extern __shared__ __align__(128) uint8_t sm[];
@@ -190,8 +188,8 @@ __global__ void __launch_bounds__(ROWS * Tile<LA, LB, C>::GROUPS, 1)
   fence_before();
   __syncthreads();
   fence_after();
-  if (!wait_parity(ctrl + 8, 0, WAIT_POLLS)) atomicAdd(&g_ntt_tc_wait_errors, 1u);
-  Group gr = make_group(sm, S::O_CTRL, ctrl + 16, COLS, &g_ntt_tc_wait_errors);
+  if (!wait_parity(ctrl + 8, 0, WAIT_POLLS)) report_wait(waits);
+  Group gr = make_group(sm, S::O_CTRL, ctrl + 16, COLS, waits);
 
   const int gi = threadIdx.x / ROWS, tid = threadIdx.x % ROWS;
   uint8_t *mine = sm + S::O_GROUP + gi * S::PER_GROUP;
@@ -286,7 +284,7 @@ struct FusedTile {
 template <int LA, int LB, int C>
 __global__ void __launch_bounds__(ROWS * FusedTile<LA, LB, C>::GROUPS, 1)
     fused_kernel(T *out, const FusedGeom g, uint64_t tiles, const T *__restrict__ itw, const T *__restrict__ ftw,
-                 const T *__restrict__ ctab_t, const T *__restrict__ ftw_t, const __grid_constant__ CUtensorMap map) {
+                 const T *__restrict__ ctab_t, const T *__restrict__ ftw_t, const __grid_constant__ CUtensorMap map, uint32_t *waits) {
   using S = Tile<LA, LB, C>;
   using U = FusedTile<LA, LB, C>;
   constexpr int K = S::K, RA = S::RA, RB = S::RB;
@@ -317,8 +315,8 @@ __global__ void __launch_bounds__(ROWS * FusedTile<LA, LB, C>::GROUPS, 1)
   fence_before();
   __syncthreads();
   fence_after();
-  if (!wait_parity(ctrl + 8, 0, WAIT_POLLS)) atomicAdd(&g_ntt_tc_wait_errors, 1u);
-  Group gr = make_group(sm, U::O_CTRL, ctrl + 16, COLS, &g_ntt_tc_wait_errors);
+  if (!wait_parity(ctrl + 8, 0, WAIT_POLLS)) report_wait(waits);
+  Group gr = make_group(sm, U::O_CTRL, ctrl + 16, COLS, waits);
 
   const int gi = threadIdx.x / ROWS, tid = threadIdx.x % ROWS;
   uint8_t *mine = sm + U::O_GROUP + gi * U::PER_GROUP;
@@ -412,7 +410,7 @@ static int launch(T *out, const PassGeom &g, uint64_t tiles, const T *tw, bool i
   ZKB_TRY(current_context(&ctx));
   ZKB_CHECK_CUDA(cudaFuncSetAttribute(pass_kernel<LA, LB, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
   const unsigned grid = (unsigned)std::min<uint64_t>(ctx->sm_count, tiles);
-  ZKB_LAUNCH("ntt_pass_tc", s, pass_kernel<LA, LB, C><<<grid, ROWS * S::GROUPS, S::SMEM, s>>>(out, g, tiles, tw, inverse ? 1 : 0, scale, map));
+  ZKB_LAUNCH("ntt_pass_tc", s, pass_kernel<LA, LB, C><<<grid, ROWS * S::GROUPS, S::SMEM, s>>>(out, g, tiles, tw, inverse ? 1 : 0, scale, map, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -436,7 +434,7 @@ static int launch_fused(T *out, const FusedGeom &g, uint64_t tiles, const T *itw
   ZKB_TRY(current_context(&ctx));
   ZKB_CHECK_CUDA(cudaFuncSetAttribute(fused_kernel<LA, LB, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, U::SMEM));
   const unsigned grid = (unsigned)std::min<uint64_t>(ctx->sm_count, tiles);
-  ZKB_LAUNCH("lde_fused_tc", s, fused_kernel<LA, LB, C><<<grid, ROWS * U::GROUPS, U::SMEM, s>>>(out, g, tiles, itw, ftw, ctab_t, ftw_t, map));
+  ZKB_LAUNCH("lde_fused_tc", s, fused_kernel<LA, LB, C><<<grid, ROWS * U::GROUPS, U::SMEM, s>>>(out, g, tiles, itw, ftw, ctab_t, ftw_t, map, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -448,14 +446,6 @@ int fused(int K, T *out, const FusedGeom &g, uint64_t tiles, const T *itw, const
     case 8: return launch_fused<4, 4, 8>(out, g, tiles, itw, ftw, ctab_t, ftw_t, map, s);
     default: set_error("internal: fused LDE pass of %d bits", K); return ZKB_ERR_INTERNAL;
   }
-}
-
-int wait_errors(uint32_t *count) {
-  uint32_t v = 0, zero = 0;
-  ZKB_CHECK_CUDA(cudaMemcpyFromSymbol(&v, g_ntt_tc_wait_errors, sizeof v));
-  ZKB_CHECK_CUDA(cudaMemcpyToSymbol(g_ntt_tc_wait_errors, &zero, sizeof zero));
-  *count = v;
-  return ZKB_OK;
 }
 
 }  // namespace ntt_tc

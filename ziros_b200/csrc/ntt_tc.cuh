@@ -16,7 +16,6 @@ int pass(int K, uint64_t *out, const PassGeom &g, uint64_t tiles, const uint64_t
 // The fused LDE middle over `tiles` tiles, tables as lde_fused_kernel's.
 int fused(int K, uint64_t *out, const FusedGeom &g, uint64_t tiles, const uint64_t *itw, const uint64_t *ftw,
           const uint64_t *ctab_t, const uint64_t *ftw_t, const CUtensorMap &map, cudaStream_t s);
-int wait_errors(uint32_t *count);
 
 }  // namespace ntt_tc
 }  // namespace zkb

@@ -250,7 +250,7 @@ __device__ __forceinline__ void ntt_pass_tile(const typename F::T *in, typename 
     T x[R1];
     if (active) {
       if constexpr (TMA_IN) {
-        if (!mbar_wait(bar, 0, TMA_WAIT_LIMIT)) atomicExch(err, 1u);
+        if (!mbar_wait(bar, 0, TMA_WAIT_LIMIT)) report_wait(err);
         const T *tp = sm + i * C + c;
 #pragma unroll
         for (int j = 0; j < R1; j++) x[j] = tp[j * R2 * C];
@@ -372,7 +372,7 @@ __device__ __forceinline__ void lde_fused_tile(const typename F::T *in, typename
     T x[R1];
     if (active) {
       if constexpr (TMA_IN) {
-        if (!mbar_wait(bar, 0, TMA_WAIT_LIMIT)) atomicExch(err, 1u);
+        if (!mbar_wait(bar, 0, TMA_WAIT_LIMIT)) report_wait(err);
         const T *tp = sm + i * C + c;
 #pragma unroll
         for (int j = 0; j < R1; j++) x[j] = tp[j * R2 * C];

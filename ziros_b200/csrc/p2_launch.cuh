@@ -48,8 +48,6 @@ int fri_fold_hash(const uint32_t *e, uint32_t *out, uint64_t n_leaves, int log_o
                   const uint32_t *itw, uint32_t *digests, const P2Params<BabyBear, 16> &p, const char *name,
                   cudaStream_t s);
 int permute(uint32_t *states, uint64_t n, const P2Params<BabyBear, 16> &p, cudaStream_t s);
-// Waits that gave up since the last call (resets the count).
-int wait_errors(uint32_t *count);
 
 }  // namespace p2t
 
@@ -72,7 +70,6 @@ int mt_compress(const mt::CompJob *d_jobs, int n, uint64_t total, const P2Params
                 cudaStream_t s);
 template <int W>
 int permute(uint64_t *states, uint64_t n, const P2Params<Goldilocks, W> &p, cudaStream_t s);
-int wait_errors(uint32_t *count);
 
 }  // namespace p2g
 

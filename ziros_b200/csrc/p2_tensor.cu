@@ -21,8 +21,6 @@
 
 namespace zkb {
 
-__device__ uint32_t g_p2t_wait_errors;
-
 namespace p2t {
 
 constexpr int THREADS = GROUP * MAX_GROUPS;
@@ -101,12 +99,12 @@ __device__ __forceinline__ void prefetch(const void *p) { asm volatile("prefetch
 template <bool COMBINE>
 __global__ void __launch_bounds__(THREADS)
     leaf_kernel(const MatList ml, uint64_t height, uint32_t *__restrict__ digests,
-                const __grid_constant__ P2Params<BabyBear, 16> p, const uint4 *__restrict__ apow,
+                const __grid_constant__ P2Params<BabyBear, 16> p, uint32_t *waits, const uint4 *__restrict__ apow,
                 uint4 *__restrict__ comb, bool vec) {
   extern __shared__ __align__(128) uint8_t sm[];
   const uint64_t width = ml.col_start[ml.n];
   const int rem = (int)((width - 1) % 8) + 1;
-  Group g = setup(sm, p, SPONGE, rem, &g_p2t_wait_errors);
+  Group g = setup(sm, p, SPONGE, rem, waits);
   const uint64_t tiles = (height + GROUP - 1) / GROUP;
   P2T_TILES(t, tiles) {
     uint64_t row = t * GROUP + threadIdx.x % GROUP;
@@ -149,11 +147,11 @@ template <bool COMBINE>
 __global__ void __launch_bounds__(THREADS)
     slab_kernel(const uint32_t *__restrict__ mat, uint64_t stride, uint64_t c0, uint64_t ncols, uint64_t height,
                 uint32_t *__restrict__ carry, int first, int last, uint32_t *__restrict__ digests,
-                const __grid_constant__ P2Params<BabyBear, 16> p, const uint4 *__restrict__ apow,
+                const __grid_constant__ P2Params<BabyBear, 16> p, uint32_t *waits, const uint4 *__restrict__ apow,
                 uint4 *__restrict__ comb, bool vec) {
   extern __shared__ __align__(128) uint8_t sm[];
   const int rem = (int)((ncols - 1) % 8) + 1;
-  Group g = setup(sm, p, SPONGE, rem, &g_p2t_wait_errors);
+  Group g = setup(sm, p, SPONGE, rem, waits);
   const uint64_t tiles = (height + GROUP - 1) / GROUP;
   P2T_TILES(t, tiles) {
     uint64_t row = t * GROUP + threadIdx.x % GROUP;
@@ -220,9 +218,9 @@ __device__ __forceinline__ void load16(uint32_t (&x)[16], const uint32_t *from) 
 // next[i] = compress(prev[2i], prev[2i+1]); with inj, compress(that, i < inj_h ? inj[i] : 0).
 __global__ void __launch_bounds__(THREADS)
     compress_kernel(const uint32_t *__restrict__ prev, uint32_t *__restrict__ next, uint64_t n_out,
-                    const uint32_t *__restrict__ inj, uint64_t inj_h, const __grid_constant__ P2Params<BabyBear, 16> p) {
+                    const uint32_t *__restrict__ inj, uint64_t inj_h, const __grid_constant__ P2Params<BabyBear, 16> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
-  Group g = setup(sm, p, STATE16, 8, &g_p2t_wait_errors);
+  Group g = setup(sm, p, STATE16, 8, waits);
   const uint64_t tiles = (n_out + GROUP - 1) / GROUP;
   P2T_TILES(t, tiles) {
     uint64_t i = t * GROUP + threadIdx.x % GROUP;
@@ -250,11 +248,11 @@ __global__ void __launch_bounds__(THREADS)
 // Leaf sponges of many matrices: tile t belongs to the last job whose first tile is <= t.
 __global__ void __launch_bounds__(THREADS)
     mt_leaf_kernel(const mt::LeafJob *__restrict__ jobs, int n_jobs, uint64_t tiles,
-                   const __grid_constant__ P2Params<BabyBear, 16> p) {
+                   const __grid_constant__ P2Params<BabyBear, 16> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
   uint64_t *starts = reinterpret_cast<uint64_t *>(sm + mt_smem(SPONGE_ANY, 0));
   for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].tile_start;
-  Group g = setup(sm, p, SPONGE_ANY, 8, &g_p2t_wait_errors);
+  Group g = setup(sm, p, SPONGE_ANY, 8, waits);
   P2T_TILES(t, tiles) {
     const int j = mt::find_job(starts, n_jobs, t);
     const uint64_t rows = jobs[j].rows, width = jobs[j].width;
@@ -282,11 +280,11 @@ __global__ void __launch_bounds__(THREADS)
 // One level of many trees: each thread finds its own job.
 __global__ void __launch_bounds__(THREADS)
     mt_compress_kernel(const mt::CompJob *__restrict__ jobs, int n_jobs, uint64_t total,
-                       const __grid_constant__ P2Params<BabyBear, 16> p) {
+                       const __grid_constant__ P2Params<BabyBear, 16> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
   uint64_t *starts = reinterpret_cast<uint64_t *>(sm + mt_smem(STATE16, 0));
   for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].start;
-  Group g = setup(sm, p, STATE16, 8, &g_p2t_wait_errors);
+  Group g = setup(sm, p, STATE16, 8, waits);
   const uint64_t tiles = (total + GROUP - 1) / GROUP;
   P2T_TILES(t, tiles) {
     uint64_t q = t * GROUP + threadIdx.x % GROUP;
@@ -309,9 +307,9 @@ template <bool FOLD>
 __global__ void __launch_bounds__(THREADS)
     fri_kernel(const uint32_t *__restrict__ e, uint32_t *__restrict__ out, uint64_t n_leaves, int log_out,
                const Ext4Params prm, const uint32_t *__restrict__ itw, uint32_t *__restrict__ digests,
-               const __grid_constant__ P2Params<BabyBear, 16> p) {
+               const __grid_constant__ P2Params<BabyBear, 16> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
-  Group g = setup(sm, p, SPONGE, 8, &g_p2t_wait_errors);
+  Group g = setup(sm, p, SPONGE, 8, waits);
   const uint64_t tiles = (n_leaves + GROUP - 1) / GROUP;
   P2T_TILES(t, tiles) {
     uint64_t j = t * GROUP + threadIdx.x % GROUP;
@@ -343,9 +341,9 @@ __global__ void __launch_bounds__(THREADS)
 }
 
 __global__ void __launch_bounds__(THREADS)
-    permute_kernel(uint32_t *__restrict__ states, uint64_t n, bool vec, const __grid_constant__ P2Params<BabyBear, 16> p) {
+    permute_kernel(uint32_t *__restrict__ states, uint64_t n, bool vec, const __grid_constant__ P2Params<BabyBear, 16> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
-  Group g = setup(sm, p, PERM16, 8, &g_p2t_wait_errors);
+  Group g = setup(sm, p, PERM16, 8, waits);
   const uint64_t tiles = (n + GROUP - 1) / GROUP;
   P2T_TILES(t, tiles) {
     uint64_t i = t * GROUP + threadIdx.x % GROUP;
@@ -411,10 +409,10 @@ int hash_rows(const MatList &ml, uint64_t height, uint32_t *digests, const P2Par
   const bool vec = ml.n == 1 && width % 4 == 0 && ((uintptr_t)ml.ptr[0] & 15) == 0;
   if (comb) {
     ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(leaf_kernel<true>));
-    ZKB_LAUNCH(name, s, leaf_kernel<true><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, apow, comb, vec));
+    ZKB_LAUNCH(name, s, leaf_kernel<true><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, ctx->wait_word, apow, comb, vec));
   } else {
     ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(leaf_kernel<false>));
-    ZKB_LAUNCH(name, s, leaf_kernel<false><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, apow, comb, vec));
+    ZKB_LAUNCH(name, s, leaf_kernel<false><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, ctx->wait_word, apow, comb, vec));
   }
   return ZKB_OK;
 }
@@ -429,10 +427,10 @@ int hash_slab(const uint32_t *mat, uint64_t stride, uint64_t c0, uint64_t ncols,
   const bool vec = stride % 4 == 0 && c0 % 4 == 0 && ncols % 4 == 0 && ((uintptr_t)mat & 15) == 0;
   if (apow) {
     ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(slab_kernel<true>));
-    ZKB_LAUNCH(name, s, slab_kernel<true><<<sh.grid, sh.threads, smem, s>>>(mat, stride, c0, ncols, height, carry, first, last, digests, p, apow, comb, vec));
+    ZKB_LAUNCH(name, s, slab_kernel<true><<<sh.grid, sh.threads, smem, s>>>(mat, stride, c0, ncols, height, carry, first, last, digests, p, ctx->wait_word, apow, comb, vec));
   } else {
     ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(slab_kernel<false>));
-    ZKB_LAUNCH(name, s, slab_kernel<false><<<sh.grid, sh.threads, smem, s>>>(mat, stride, c0, ncols, height, carry, first, last, digests, p, apow, comb, vec));
+    ZKB_LAUNCH(name, s, slab_kernel<false><<<sh.grid, sh.threads, smem, s>>>(mat, stride, c0, ncols, height, carry, first, last, digests, p, ctx->wait_word, apow, comb, vec));
   }
   return ZKB_OK;
 }
@@ -444,7 +442,7 @@ int compress(const uint32_t *prev, uint32_t *next, uint64_t n_out, const uint32_
   const Shape sh = shape((n_out + GROUP - 1) / GROUP, 1, ctx->sm_count);
   const size_t smem = smem_bytes(STATE16);
   ZKB_TRY(smem_limit<smem_bytes(STATE16)>(compress_kernel));
-  ZKB_LAUNCH(name, s, compress_kernel<<<sh.grid, sh.threads, smem, s>>>(prev, next, n_out, inj, inj_h, p));
+  ZKB_LAUNCH(name, s, compress_kernel<<<sh.grid, sh.threads, smem, s>>>(prev, next, n_out, inj, inj_h, p, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -456,7 +454,7 @@ int mt_leaf(const mt::LeafJob *d_jobs, int n, uint64_t tiles, uint64_t perms, co
   ZKB_REQUIRE(n <= mt::MAX_JOBS, "internal: %d trees in one launch", n);
   const size_t smem = mt_smem(SPONGE_ANY, n);
   ZKB_TRY(smem_limit<mt_smem(SPONGE_ANY, mt::MAX_JOBS)>(mt_leaf_kernel));
-  ZKB_LAUNCH(name, s, mt_leaf_kernel<<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, tiles, p));
+  ZKB_LAUNCH(name, s, mt_leaf_kernel<<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, tiles, p, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -468,7 +466,7 @@ int mt_compress(const mt::CompJob *d_jobs, int n, uint64_t total, const P2Params
   ZKB_REQUIRE(n <= mt::MAX_JOBS, "internal: %d trees in one launch", n);
   const size_t smem = mt_smem(STATE16, n);
   ZKB_TRY(smem_limit<mt_smem(STATE16, mt::MAX_JOBS)>(mt_compress_kernel));
-  ZKB_LAUNCH(name, s, mt_compress_kernel<<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, total, p));
+  ZKB_LAUNCH(name, s, mt_compress_kernel<<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, total, p, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -481,10 +479,10 @@ int fri_fold_hash(const uint32_t *e, uint32_t *out, uint64_t n_leaves, int log_o
   const size_t smem = smem_bytes(SPONGE);
   if (prm) {
     ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(fri_kernel<true>));
-    ZKB_LAUNCH(name, s, fri_kernel<true><<<sh.grid, sh.threads, smem, s>>>(e, out, n_leaves, log_out, *prm, itw, digests, p));
+    ZKB_LAUNCH(name, s, fri_kernel<true><<<sh.grid, sh.threads, smem, s>>>(e, out, n_leaves, log_out, *prm, itw, digests, p, ctx->wait_word));
   } else {
     ZKB_TRY(smem_limit<smem_bytes(SPONGE)>(fri_kernel<false>));
-    ZKB_LAUNCH(name, s, fri_kernel<false><<<sh.grid, sh.threads, smem, s>>>(e, out, n_leaves, log_out, Ext4Params{}, itw, digests, p));
+    ZKB_LAUNCH(name, s, fri_kernel<false><<<sh.grid, sh.threads, smem, s>>>(e, out, n_leaves, log_out, Ext4Params{}, itw, digests, p, ctx->wait_word));
   }
   return ZKB_OK;
 }
@@ -496,15 +494,7 @@ int permute(uint32_t *states, uint64_t n, const P2Params<BabyBear, 16> &p, cudaS
   const size_t smem = smem_bytes(PERM16);
   ZKB_TRY(smem_limit<smem_bytes(PERM16)>(permute_kernel));
   const bool vec = ((uintptr_t)states & 15) == 0;
-  ZKB_LAUNCH("p2_permute", s, permute_kernel<<<sh.grid, sh.threads, smem, s>>>(states, n, vec, p));
-  return ZKB_OK;
-}
-
-int wait_errors(uint32_t *count) {
-  uint32_t v = 0, zero = 0;
-  ZKB_CHECK_CUDA(cudaMemcpyFromSymbol(&v, g_p2t_wait_errors, sizeof v));
-  ZKB_CHECK_CUDA(cudaMemcpyToSymbol(g_p2t_wait_errors, &zero, sizeof zero));
-  *count = v;
+  ZKB_LAUNCH("p2_permute", s, permute_kernel<<<sh.grid, sh.threads, smem, s>>>(states, n, vec, p, ctx->wait_word));
   return ZKB_OK;
 }
 

@@ -504,7 +504,7 @@ __device__ __forceinline__ Group setup(uint8_t *sm, const P2Params<BabyBear, 16>
     reinterpret_cast<uint4 *>(sm + S_C)[t] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x < 32) tmem_alloc(ctrl, tmem_cols(groups));
   __syncthreads();
-  if (!wait_parity(tables, 0, WAIT_POLLS)) atomicAdd(err, 1u);
+  if (!wait_parity(tables, 0, WAIT_POLLS)) report_wait(err);
   put_constants(sm, p);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   fence_before();

@@ -15,8 +15,6 @@
 
 namespace zkb {
 
-__device__ uint32_t g_p2g_wait_errors;
-
 namespace p2g {
 
 template <int W>
@@ -100,9 +98,9 @@ __device__ __forceinline__ void sponge(Group &g, uint64_t width, Load load) {
 template <int W>
 __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     leaf_kernel(const MatList ml, uint64_t height, uint64_t *__restrict__ digests,
-                const __grid_constant__ P2Params<Goldilocks, W> p, bool vec) {
+                const __grid_constant__ P2Params<Goldilocks, W> p, uint32_t *waits, bool vec) {
   extern __shared__ __align__(128) uint8_t sm[];
-  Group g = setup<W>(sm, p, true, &g_p2g_wait_errors);
+  Group g = setup<W>(sm, p, true, waits);
   const uint64_t width = ml.col_start[ml.n], tiles = (height + GROUP - 1) / GROUP;
   P2G_TILES(t, tiles) {
     uint64_t row = t * GROUP + threadIdx.x % GROUP;
@@ -125,11 +123,11 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
 template <int W>
 __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     mt_leaf_kernel(const mt::LeafJob *__restrict__ jobs, int n_jobs, uint64_t tiles,
-                   const __grid_constant__ P2Params<Goldilocks, W> p) {
+                   const __grid_constant__ P2Params<Goldilocks, W> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
   uint64_t *starts = reinterpret_cast<uint64_t *>(sm + mt_smem<W>(0));
   for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].tile_start;
-  Group g = setup<W>(sm, p, true, &g_p2g_wait_errors);
+  Group g = setup<W>(sm, p, true, waits);
   P2G_TILES(t, tiles) {
     const int j = mt::find_job(starts, n_jobs, t);
     const uint64_t rows = jobs[j].rows, width = jobs[j].width;
@@ -159,10 +157,10 @@ __device__ __forceinline__ void enter_pair(Group &g, const uint64_t *pair) {
 template <int W>
 __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     compress_kernel(const uint64_t *__restrict__ prev, uint64_t *__restrict__ next, uint64_t n_out,
-                    const uint64_t *__restrict__ inj, uint64_t inj_h, const __grid_constant__ P2Params<Goldilocks, W> p) {
+                    const uint64_t *__restrict__ inj, uint64_t inj_h, const __grid_constant__ P2Params<Goldilocks, W> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
   constexpr int OUT = out_words<W>();
-  Group g = setup<W>(sm, p, false, &g_p2g_wait_errors);
+  Group g = setup<W>(sm, p, false, waits);
   const uint64_t tiles = (n_out + GROUP - 1) / GROUP;
   P2G_TILES(t, tiles) {
     uint64_t i = t * GROUP + threadIdx.x % GROUP;
@@ -194,12 +192,12 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
 template <int W>
 __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     mt_compress_kernel(const mt::CompJob *__restrict__ jobs, int n_jobs, uint64_t total,
-                       const __grid_constant__ P2Params<Goldilocks, W> p) {
+                       const __grid_constant__ P2Params<Goldilocks, W> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
   constexpr int OUT = out_words<W>();
   uint64_t *starts = reinterpret_cast<uint64_t *>(sm + mt_smem<W>(0));
   for (int i = threadIdx.x; i < n_jobs; i += blockDim.x) starts[i] = jobs[i].start;
-  Group g = setup<W>(sm, p, false, &g_p2g_wait_errors);
+  Group g = setup<W>(sm, p, false, waits);
   const uint64_t tiles = (total + GROUP - 1) / GROUP;
   P2G_TILES(t, tiles) {
     uint64_t q = t * GROUP + threadIdx.x % GROUP;
@@ -216,9 +214,9 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
 
 template <int W>
 __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
-    permute_kernel(uint64_t *__restrict__ states, uint64_t n, const __grid_constant__ P2Params<Goldilocks, W> p) {
+    permute_kernel(uint64_t *__restrict__ states, uint64_t n, const __grid_constant__ P2Params<Goldilocks, W> p, uint32_t *waits) {
   extern __shared__ __align__(128) uint8_t sm[];
-  Group g = setup<W>(sm, p, false, &g_p2g_wait_errors);
+  Group g = setup<W>(sm, p, false, waits);
   const uint64_t tiles = (n + GROUP - 1) / GROUP;
   P2G_TILES(t, tiles) {
     uint64_t i = t * GROUP + threadIdx.x % GROUP;
@@ -289,7 +287,7 @@ int hash_rows(const MatList &ml, uint64_t height, uint64_t *digests, const P2Par
   const size_t smem = Shape<W>::SMEM;
   const bool vec = ml.n == 1 && ml.width[0] % 2 == 0 && ((uintptr_t)ml.ptr[0] & 15) == 0;
   ZKB_TRY(smem_limit<Shape<W>::SMEM>(leaf_kernel<W>));
-  ZKB_LAUNCH(name, s, leaf_kernel<W><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, vec));
+  ZKB_LAUNCH(name, s, leaf_kernel<W><<<sh.grid, sh.threads, smem, s>>>(ml, height, digests, p, ctx->wait_word, vec));
   return ZKB_OK;
 }
 
@@ -301,7 +299,7 @@ int compress(const uint64_t *prev, uint64_t *next, uint64_t n_out, const uint64_
   const Launch sh = shape<W>((n_out + GROUP - 1) / GROUP, 1, ctx->sm_count);
   const size_t smem = Shape<W>::SMEM;
   ZKB_TRY(smem_limit<Shape<W>::SMEM>(compress_kernel<W>));
-  ZKB_LAUNCH(name, s, compress_kernel<W><<<sh.grid, sh.threads, smem, s>>>(prev, next, n_out, inj, inj_h, p));
+  ZKB_LAUNCH(name, s, compress_kernel<W><<<sh.grid, sh.threads, smem, s>>>(prev, next, n_out, inj, inj_h, p, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -314,7 +312,7 @@ int mt_leaf(const mt::LeafJob *d_jobs, int n, uint64_t tiles, uint64_t perms, co
   ZKB_REQUIRE(n <= mt::MAX_JOBS, "internal: %d trees in one launch", n);
   const size_t smem = mt_smem<W>(n);
   ZKB_TRY(smem_limit<mt_smem<W>(mt::MAX_JOBS)>(mt_leaf_kernel<W>));
-  ZKB_LAUNCH(name, s, mt_leaf_kernel<W><<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, tiles, p));
+  ZKB_LAUNCH(name, s, mt_leaf_kernel<W><<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, tiles, p, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -327,7 +325,7 @@ int mt_compress(const mt::CompJob *d_jobs, int n, uint64_t total, const P2Params
   ZKB_REQUIRE(n <= mt::MAX_JOBS, "internal: %d trees in one launch", n);
   const size_t smem = mt_smem<W>(n);
   ZKB_TRY(smem_limit<mt_smem<W>(mt::MAX_JOBS)>(mt_compress_kernel<W>));
-  ZKB_LAUNCH(name, s, mt_compress_kernel<W><<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, total, p));
+  ZKB_LAUNCH(name, s, mt_compress_kernel<W><<<sh.grid, sh.threads, smem, s>>>(d_jobs, n, total, p, ctx->wait_word));
   return ZKB_OK;
 }
 
@@ -338,15 +336,7 @@ int permute(uint64_t *states, uint64_t n, const P2Params<Goldilocks, W> &p, cuda
   const Launch sh = shape<W>((n + GROUP - 1) / GROUP, 1, ctx->sm_count);
   const size_t smem = Shape<W>::SMEM;
   ZKB_TRY(smem_limit<Shape<W>::SMEM>(permute_kernel<W>));
-  ZKB_LAUNCH("p2_permute", s, permute_kernel<W><<<sh.grid, sh.threads, smem, s>>>(states, n, p));
-  return ZKB_OK;
-}
-
-int wait_errors(uint32_t *count) {
-  uint32_t v = 0, zero = 0;
-  ZKB_CHECK_CUDA(cudaMemcpyFromSymbol(&v, g_p2g_wait_errors, sizeof v));
-  ZKB_CHECK_CUDA(cudaMemcpyToSymbol(g_p2g_wait_errors, &zero, sizeof zero));
-  *count = v;
+  ZKB_LAUNCH("p2_permute", s, permute_kernel<W><<<sh.grid, sh.threads, smem, s>>>(states, n, p, ctx->wait_word));
   return ZKB_OK;
 }
 

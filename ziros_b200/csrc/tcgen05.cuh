@@ -4,6 +4,8 @@
 #pragma once
 #include <cstdint>
 
+#include "common.cuh"
+
 namespace zkb {
 namespace tc {
 
@@ -119,7 +121,7 @@ struct Group {
   bool lead;        // this is the warp that issues the products (warp-uniform)
   uint32_t one;     // set in one lane of it
   uint32_t polls;   // limit of a wait (0 once one has run out)
-  uint32_t *err;
+  uint32_t *err;    // DeviceContext::wait_word
 };
 
 // D columns += (or =) A columns x the K step of 32 bytes at shared offset `off` (N rows of a matrix
@@ -144,7 +146,7 @@ __device__ __forceinline__ void finish(Group &g) {
         "r"(g.one)
         : "memory");
   if (!wait_parity(g.mbar, g.phase, g.polls)) {
-    if (g.polls) atomicAdd(g.err, 1u);
+    if (g.polls) report_wait(g.err);
     g.polls = 0;
   }
   g.phase ^= 1;
