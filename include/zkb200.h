@@ -89,8 +89,9 @@ ZKB_API int zkb_get_thresholds(zkb_thresholds *thresholds_out);
  * next `count` device allocations fail as out of memory; kind 2: the next `count` stream
  * waits report an expired deadline (after the work has finished). */
 ZKB_API int zkb_debug_inject_fault(int kind, int count);
-/* For tests: one block whose wait for a tensor-core product that nothing issues gives up after
- * `polls` (1..4096) polls.  No counterpart in the reference. */
+/* For tests: a block whose 128 threads' waits for a tensor-core product that nothing issues give up
+ * after `polls` (1..4096) polls, and one whose wait for its tables does (129 waits that gave up).  No
+ * counterpart in the reference. */
 ZKB_API int zkb_debug_wait_expiry(uint32_t polls, void *stream);
 /* Number of device allocations (stream-ordered pool or cudaMalloc) the library has
  * made in this process.  Tests read it around a call to check that the call allocated

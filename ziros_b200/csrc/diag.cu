@@ -63,7 +63,7 @@ int measure_mul_peak(int field, double *mul_per_s) {
 }
 
 // A group of the hashing kernels waits for a product that nothing issued, `polls` polls long (about 4 us
-// each), then goes on to a second layer and ends.
+// each), then goes on to a second layer, drains and ends.
 __global__ void __launch_bounds__(128) wait_expiry_kernel(uint32_t polls, uint32_t *waits) {
   __shared__ __align__(16) uint8_t sm[16];
   const uint32_t mbar = (uint32_t)__cvta_generic_to_shared(sm) + 8;
@@ -78,12 +78,32 @@ __global__ void __launch_bounds__(128) wait_expiry_kernel(uint32_t polls, uint32
   g.polls = polls;
   tc::finish(g);
   tc::finish(g);
+  g.one = threadIdx.x == 0;
+  tc::drain(g, polls);
+}
+
+// A block whose tables never come ends by itself and gives its TMEM back.
+__global__ void __launch_bounds__(128) tables_expiry_kernel(uint32_t polls, uint32_t *waits) {
+  __shared__ __align__(16) uint8_t sm[16];
+  const uint32_t slot = (uint32_t)__cvta_generic_to_shared(sm), mbar = slot + 8;
+  if (threadIdx.x == 0) {
+    tc::init_barrier(mbar);
+    tc::init_fence();
+  }
+  if (threadIdx.x < 32) tc::tmem_alloc(slot, 128);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  tc::tables_or_exit(mbar, sm, 128, waits, polls);
+  report_wait(waits);  // not reached
+  if (threadIdx.x < 32) tc::tmem_free(*reinterpret_cast<const volatile uint32_t *>(sm), 128);
 }
 
 int debug_wait_expiry(uint32_t polls, cudaStream_t s) {
   DeviceContext *ctx;
   ZKB_TRY(current_context(&ctx));
   ZKB_LAUNCH("debug_wait_expiry", s, wait_expiry_kernel<<<1, 128, 0, s>>>(polls, ctx->wait_word));
+  ZKB_LAUNCH("debug_wait_expiry", s, tables_expiry_kernel<<<1, 128, 0, s>>>(polls, ctx->wait_word));
   return ZKB_OK;
 }
 

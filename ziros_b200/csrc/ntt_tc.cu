@@ -114,12 +114,17 @@ __device__ __forceinline__ void tile_copy(const T *tile, const CUtensorMap *map,
       "l"(map), "r"(x), "r"(low), "r"(0), "r"(0), "r"(high), "r"(mbar)
       : "memory");
 }
-__device__ __forceinline__ void group_wait(Group &g, uint32_t mbar, uint32_t &phase) {
-  if (!wait_parity(mbar, phase, g.polls)) {
+// The group's tile has come.  `in_flight`: this thread has started its copy; when the wait gives up (or one
+// before it has), that thread waits for the copy once more, so that none is under way when the block ends.
+__device__ __forceinline__ void group_wait(Group &g, uint32_t mbar, uint32_t &phase, bool &in_flight) {
+  if (wait_parity(mbar, phase, g.polls)) {
+    phase ^= 1;
+  } else {
     if (g.polls) report_wait(g.err);
     g.polls = 0;
+    if (in_flight) wait_parity(mbar, phase, WAIT_POLLS);
   }
-  phase ^= 1;
+  in_flight = false;
 }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void group_sync(const Group &g) { asm volatile("bar.sync %0, 128;" ::"r"(g.bar) : "memory"); }
@@ -188,7 +193,7 @@ __global__ void __launch_bounds__(ROWS * Tile<LA, LB, C>::GROUPS, 1)
   fence_before();
   __syncthreads();
   fence_after();
-  if (!wait_parity(ctrl + 8, 0, WAIT_POLLS)) report_wait(waits);
+  tables_or_exit(ctrl + 8, sm + S::O_CTRL, 512, waits);
   Group gr = make_group(sm, S::O_CTRL, ctrl + 16, COLS, waits);
 
   const int gi = threadIdx.x / ROWS, tid = threadIdx.x % ROWS;
@@ -197,7 +202,9 @@ __global__ void __launch_bounds__(ROWS * Tile<LA, LB, C>::GROUPS, 1)
   T *tw_b = reinterpret_cast<T *>(mine + S::BYTES);
   const uint32_t load = loads + 8 * gi;
   const uint64_t stride = (uint64_t)gridDim.x * S::GROUPS;
+  bool in_flight = false;
   auto fetch = [&](uint64_t t) {  // one thread: the copy of tile t
+    in_flight = true;
     const uint32_t chunk = (uint32_t)(t % g.chunks_per_row);
     const uint64_t rest = t / g.chunks_per_row;
     const uint32_t grp = (uint32_t)(rest % g.groups), blk = (uint32_t)(rest / g.groups);
@@ -218,7 +225,7 @@ __global__ void __launch_bounds__(ROWS * Tile<LA, LB, C>::GROUPS, 1)
       for (int e = tid; e < S::ROWS_T; e += ROWS) tw_b[e] = tw[((uint64_t)i_low * e) << (g.L - hi)];
       staged = i_low;  // visible after the barriers of phase A
     }
-    group_wait(gr, load, phase);
+    group_wait(gr, load, phase, in_flight);
     // ---- phase A: over j of rows j * RB + i; outputs in place, i's low bits xored with f1's so that neither
     // phase's warps meet a bank twice (the xor stays inside the batch)
 #pragma unroll 1
@@ -250,13 +257,14 @@ __global__ void __launch_bounds__(ROWS * Tile<LA, LB, C>::GROUPS, 1)
           },
           [&] {
             // every thread of the group has read its last inputs: the tile's memory is free
-            if (b == S::NB - 1 && tid == 0 && t + stride < tiles) {
+            if (b == S::NB - 1 && tid == 0 && t + stride < tiles && gr.polls) {
               proxy_fence();
               fetch(t + stride);
             }
           });
     }
   }
+  drain(gr);
   st_wait();
   fence_before();
   __syncthreads();
@@ -315,7 +323,7 @@ __global__ void __launch_bounds__(ROWS * FusedTile<LA, LB, C>::GROUPS, 1)
   fence_before();
   __syncthreads();
   fence_after();
-  if (!wait_parity(ctrl + 8, 0, WAIT_POLLS)) report_wait(waits);
+  tables_or_exit(ctrl + 8, sm + U::O_CTRL, 512, waits);
   Group gr = make_group(sm, U::O_CTRL, ctrl + 16, COLS, waits);
 
   const int gi = threadIdx.x / ROWS, tid = threadIdx.x % ROWS;
@@ -324,7 +332,9 @@ __global__ void __launch_bounds__(ROWS * FusedTile<LA, LB, C>::GROUPS, 1)
   T *cf = reinterpret_cast<T *>(mine + 2 * S::BYTES), *tw_b = cf + S::ROWS_T;
   const uint32_t load = loads + 8 * gi;
   const uint64_t stride = (uint64_t)gridDim.x * U::GROUPS, first = (uint64_t)gi * gridDim.x + blockIdx.x;
+  bool in_flight = false;
   auto fetch = [&](uint64_t t) {
+    in_flight = true;
     tile_copy(tile, &map, (int)(t % g.chunks_per_row) * C, 0, (int)(t / g.chunks_per_row), load, S::BYTES);
   };
   if (tid == 0 && first < tiles) fetch(first);
@@ -338,7 +348,7 @@ __global__ void __launch_bounds__(ROWS * FusedTile<LA, LB, C>::GROUPS, 1)
     group_sync(gr);  // the last tile's uses of the tables are over
     for (int e = tid; e < S::ROWS_T; e += ROWS) tw_b[e] = ftw_t[((size_t)m_lo << K) + e];
     factors(0);
-    group_wait(gr, load, phase);
+    group_wait(gr, load, phase, in_flight);
     // ---- inverse pass: phase A in place, phase B into the coefficients, index e = f1 + RA f2
 #pragma unroll 1
     for (int b = 0; b < S::NA; b++) {
@@ -385,7 +395,7 @@ __global__ void __launch_bounds__(ROWS * FusedTile<LA, LB, C>::GROUPS, 1)
               if (ok) p[(size_t)(__brev(f) >> (32 - LB)) * rs] = F::canon(x);
             },
             [&] {
-              if (last && b == S::NB - 1 && tid == 0 && t + stride < tiles) {
+              if (last && b == S::NB - 1 && tid == 0 && t + stride < tiles && gr.polls) {
                 proxy_fence();
                 fetch(t + stride);
               }
@@ -393,6 +403,7 @@ __global__ void __launch_bounds__(ROWS * FusedTile<LA, LB, C>::GROUPS, 1)
       }
     }
   }
+  drain(gr);
   st_wait();
   fence_before();
   __syncthreads();

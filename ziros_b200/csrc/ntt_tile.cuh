@@ -148,9 +148,8 @@ __device__ __forceinline__ void dif_reg(typename F::T (&x)[1 << LR], const Small
 // tensor map views a column segment as 5 dimensions (column, row bits below the pass,
 // the pass's bits in two parts of at most 8, the bits above it with the transform index)
 // and the box is C columns x 2^K rows, so row r of the tile lands at r * C.  Completion is
-// tracked by an mbarrier; every wait gives up after a bounded number of polls and raises an
-// error word instead of hanging.
-constexpr uint32_t TMA_WAIT_LIMIT = 1u << 24;
+// tracked by an mbarrier; every wait gives up after a bounded number of polls and is reported
+// instead of hanging.
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -173,6 +172,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
         : "r"(smem_addr(bar)), "r"(parity)
         : "memory");
   return done != 0;
+}
+
+// Waits for the block's tile; a wait that gives up is reported, and waits once more, so that the copy is
+// not under way when the block ends.
+static __device__ __noinline__ void tile_late(uint64_t *bar, uint32_t *err) {
+  report_wait(err);
+  mbar_wait(bar, 0, WAIT_POLLS);
+}
+__device__ __forceinline__ void tile_wait(uint64_t *bar, uint32_t *err) {
+  if (!mbar_wait(bar, 0, WAIT_POLLS)) tile_late(bar, err);
 }
 
 __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0, int c1, int c2,
@@ -250,7 +259,7 @@ __device__ __forceinline__ void ntt_pass_tile(const typename F::T *in, typename 
     T x[R1];
     if (active) {
       if constexpr (TMA_IN) {
-        if (!mbar_wait(bar, 0, TMA_WAIT_LIMIT)) report_wait(err);
+        tile_wait(bar, err);
         const T *tp = sm + i * C + c;
 #pragma unroll
         for (int j = 0; j < R1; j++) x[j] = tp[j * R2 * C];
@@ -372,7 +381,7 @@ __device__ __forceinline__ void lde_fused_tile(const typename F::T *in, typename
     T x[R1];
     if (active) {
       if constexpr (TMA_IN) {
-        if (!mbar_wait(bar, 0, TMA_WAIT_LIMIT)) report_wait(err);
+        tile_wait(bar, err);
         const T *tp = sm + i * C + c;
 #pragma unroll
         for (int j = 0; j < R1; j++) x[j] = tp[j * R2 * C];

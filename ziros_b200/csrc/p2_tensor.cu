@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(THREADS)
         comb[row] = combined(acc);
     }
   }
-  teardown(sm, SPONGE);
+  teardown(g, sm, SPONGE);
 }
 
 // The same over columns [c0, c0 + ncols) of wider rows: the last S-box outputs carried in `carry`
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(THREADS)
       }
     }
   }
-  teardown(sm, SPONGE);
+  teardown(g, sm, SPONGE);
 }
 
 __device__ __forceinline__ void load16(uint32_t (&x)[16], const uint32_t *from) {
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(THREADS)
     }
     if (live) store8(next + i * 8, o);
   }
-  teardown(sm, STATE16);
+  teardown(g, sm, STATE16);
 }
 
 // Leaf sponges of many matrices: tile t belongs to the last job whose first tile is <= t.
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(THREADS)
     leave<8>(g, o);
     if (live) store8((uint32_t *)jobs[j].digests + row * 8, o);
   }
-  teardown(sm, SPONGE_ANY);
+  teardown(g, sm, SPONGE_ANY);
 }
 
 // One level of many trees: each thread finds its own job.
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(THREADS)
     leave<8>(g, o);
     if (live) store8((uint32_t *)jobs[j].next + i * 8, o);
   }
-  teardown(sm, STATE16);
+  teardown(g, sm, STATE16);
 }
 
 // fri.cu's fold with the leaf hash of the layer it makes.
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(THREADS)
     leave<8>(g, o);
     if (live) store8(digests + j * 8, o);
   }
-  teardown(sm, SPONGE);
+  teardown(g, sm, SPONGE);
 }
 
 __global__ void __launch_bounds__(THREADS)
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(THREADS)
       for (int k = 0; k < 16; k++) states[i * 16 + k] = x[k];
     }
   }
-  teardown(sm, PERM16);
+  teardown(g, sm, PERM16);
 }
 
 // Launch shape.  A block runs up to five tiles side by side; an SM's time for k of them is

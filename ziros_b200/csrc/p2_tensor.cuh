@@ -503,8 +503,10 @@ __device__ __forceinline__ Group setup(uint8_t *sm, const P2Params<BabyBear, 16>
   for (int t = threadIdx.x; t < 8 * SLAB64 / 16; t += blockDim.x)
     reinterpret_cast<uint4 *>(sm + S_C)[t] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x < 32) tmem_alloc(ctrl, tmem_cols(groups));
+  fence_before();
   __syncthreads();
-  if (!wait_parity(tables, 0, WAIT_POLLS)) report_wait(err);
+  fence_after();
+  tables_or_exit(tables, sm + smem_tables(mode), tmem_cols(groups), err);
   put_constants(sm, p);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   fence_before();
@@ -514,7 +516,8 @@ __device__ __forceinline__ Group setup(uint8_t *sm, const P2Params<BabyBear, 16>
   st1(g.tw + COL_W + W_ONE, 1);
   return g;
 }
-__device__ __forceinline__ void teardown(uint8_t *sm, Mode mode) {
+__device__ __forceinline__ void teardown(const Group &g, uint8_t *sm, Mode mode) {
+  drain(g);
   st_wait();
   fence_before();
   __syncthreads();

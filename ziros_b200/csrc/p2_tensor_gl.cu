@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     });
     digest<W>(g, digests + row * out_words<W>(), live);
   }
-  teardown<W>(sm);
+  teardown<W>(g, sm);
 }
 
 template <int W>
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     sponge<W>(g, width, [&](uint64_t(&x)[8], uint64_t c) { load8(x, rp, c, width, vec); });
     digest<W>(g, (uint64_t *)jobs[j].digests + row * out_words<W>(), live);
   }
-  teardown<W>(sm);
+  teardown<W>(g, sm);
 }
 
 // Two digests into the state.
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     }
     digest<W>(g, next + i * OUT, live);
   }
-  teardown<W>(sm);
+  teardown<W>(g, sm);
 }
 
 template <int W>
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
     rounds<W>(g);
     digest<W>(g, (uint64_t *)jobs[j].next + i * OUT, live);
   }
-  teardown<W>(sm);
+  teardown<W>(g, sm);
 }
 
 template <int W>
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(GROUP * Shape<W>::MAX_GROUPS, 1)
       }
     }
   }
-  teardown<W>(sm);
+  teardown<W>(g, sm);
 }
 
 // Launch shape, as in p2_tensor.cu: thousands of cycles per permutation for k tiles side by side on

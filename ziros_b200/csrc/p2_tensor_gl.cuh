@@ -390,8 +390,10 @@ __device__ __forceinline__ Group setup(uint8_t *sm, const P2Params<Goldilocks, W
   for (int t = threadIdx.x; t < (S::CTRL - S::C) / 16; t += blockDim.x)
     reinterpret_cast<uint4 *>(sm + S::C)[t] = make_uint4(0, 0, 0, 0);
   if (threadIdx.x < 32) tmem_alloc(ctrl, tmem_cols<W>(groups));
+  fence_before();
   __syncthreads();
-  if (!wait_parity(tables, 0, WAIT_POLLS)) report_wait(err);
+  fence_after();
+  tables_or_exit(tables, sm + S::CTRL, tmem_cols<W>(groups), err);
   put_constants<W>(sm, p);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   fence_before();
@@ -400,7 +402,8 @@ __device__ __forceinline__ Group setup(uint8_t *sm, const P2Params<Goldilocks, W
   return make_group(sm, S::CTRL, ctrl + 16, S::COLS, err);
 }
 template <int W>
-__device__ __forceinline__ void teardown(uint8_t *sm) {
+__device__ __forceinline__ void teardown(const Group &g, uint8_t *sm) {
+  drain(g);
   st_wait();
   fence_before();
   __syncthreads();

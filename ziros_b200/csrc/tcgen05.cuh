@@ -68,7 +68,6 @@ __device__ __forceinline__ void ld_wait(uint32_t (&v)[16]) {
                  "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
 }
 
-constexpr uint32_t WAIT_POLLS = 1u << 16;
 // Waits for a phase of the mbarrier; false when `polls` polls have run out.
 __device__ __forceinline__ bool wait_parity(uint32_t mbar, uint32_t parity, uint32_t polls) {
   uint32_t done = 0;
@@ -136,21 +135,50 @@ __device__ __forceinline__ void arrive(const Group &g) {
   asm volatile("bar.sync %0, 128;" ::"r"(g.bar) : "memory");
   if (g.lead) fence_after();
 }
+// The products issued so far by the lane that has `one` set arrive on mbar when they are done.
+__device__ __forceinline__ void commit(uint32_t mbar, uint32_t one) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.u32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(mbar),
+      "r"(one)
+      : "memory");
+}
 // After the lead warp has issued the products: everyone waits for them (bounded: a wait that runs
-// out records itself and the group goes on, so every block ends).
+// out reports itself and the group goes on without waiting, so every block ends).
 __device__ __forceinline__ void finish(Group &g) {
-  if (g.lead)
-    asm volatile(
-        "{\n\t.reg .pred e;\n\tsetp.ne.u32 e, %1, 0;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(g.mbar),
-        "r"(g.one)
-        : "memory");
+  if (g.lead) commit(g.mbar, g.one);
   if (!wait_parity(g.mbar, g.phase, g.polls)) {
     if (g.polls) report_wait(g.err);
     g.polls = 0;
   }
   g.phase ^= 1;
   fence_after();
+}
+// Before the block gives its TMEM and shared memory back: where a wait gave up, products may still be under
+// way, so the lane that issued them waits for all of them on an mbarrier of its own (bounded), in the first
+// words of the tables, which nothing correct needs any more.
+static __device__ __noinline__ void drain_on(uint32_t mbar, uint32_t polls) {
+  init_barrier(mbar);
+  init_fence();
+  commit(mbar, 1);
+  wait_parity(mbar, 0, polls);
+}
+__device__ __forceinline__ void drain(const Group &g, uint32_t polls = WAIT_POLLS) {
+  if (!g.polls && g.one) drain_on(g.sm + 8 * (g.bar - 1), polls);
+}
+// The tables' copies (on the mbarrier `tables`) have landed; or they have not within the limit, and the
+// block reports that, waits once more, frees its TMEM (address at `slot`) and ends.  Every thread calls it.
+static __device__ __noinline__ void exit_without_tables(uint32_t tables, const uint8_t *slot, uint32_t cols,
+                                                        uint32_t *err, uint32_t polls) {
+  if (threadIdx.x == 0) report_wait(err);
+  wait_parity(tables, 0, polls);
+  __syncthreads();
+  if (threadIdx.x < 32) tmem_free(*reinterpret_cast<const volatile uint32_t *>(slot), cols);
+  asm volatile("exit;");
+}
+__device__ __forceinline__ void tables_or_exit(uint32_t tables, const uint8_t *slot, uint32_t cols, uint32_t *err,
+                                               uint32_t polls = WAIT_POLLS) {
+  if (!__syncthreads_and(wait_parity(tables, 0, polls))) exit_without_tables(tables, slot, cols, err, polls);
 }
 // This thread's group: `cols` TMEM columns each from the address at sm + slot on, mbarriers at
 // `mbars`, tables at `sm`.
