@@ -212,8 +212,9 @@ ZKB_API int zkb_coset_lde_batch_dev(int field, const void *d_trace, uint32_t log
  * largest NTT pass kmax index bits (1..11 BabyBear, 1..10 Goldilocks; 0 = default) and
  * the widest column chunk per CTA of the plain passes (1/4/8/16, 0 = default) and of the
  * fused middle kernel (1/4/8, 0 = default); columns beyond a multiple of the chunk take
- * narrower chunks.  Every choice gives the same output; the batched plan's
- * autotuner picks among them.  No counterpart in the reference (its Metal NTT has one
+ * a last chunk that is not full, or a narrower one.  Goldilocks passes run on the tensor
+ * cores only where no chunk is given.  Every choice gives the same output; the batched
+ * plan's autotuner picks among them and the default.  No counterpart in the reference (its Metal NTT has one
  * fixed dispatch shape, zkf-metal/src/ntt/p3_adapter.rs:78-294). */
 ZKB_API int zkb_coset_lde_tuned_dev(int field, const void *d_trace, uint32_t log_h, uint32_t width,
                                     uint32_t log_blowup, int kmax, uint32_t c_pass, uint32_t c_fused,

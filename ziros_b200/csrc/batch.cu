@@ -552,9 +552,12 @@ struct zkb_batch {
     return rc;
   }
 
+  // Goldilocks entries carry a mark: those of before the tensor-core passes, which no explicit column chunk
+  // takes, were chosen among the butterfly kernels only.
   std::string lde_key(size_t i) const {
     char k[96];
-    snprintf(k, sizeof k, "lde/%d/%u/%u/%u", spec.field, shapes[i].log_h, shapes[i].width, log_b);
+    snprintf(k, sizeof k, "lde/%d/%u/%u/%u%s", spec.field, shapes[i].log_h, shapes[i].width, log_b,
+             spec.field == FIELD_BABYBEAR ? "" : "/tc");
     return k;
   }
 
@@ -594,6 +597,9 @@ struct zkb_batch {
       }
       const uint32_t w = shapes[i].width;
       std::vector<LdeTune> cands;
+      // the default plan, which no explicit choice stands for: its passes may run on the tensor cores
+      // (BabyBear's is the first of the candidates below)
+      if (spec.field == FIELD_GOLDILOCKS) cands.push_back(LdeTune{});
       std::vector<std::vector<int>> seen_plans;
       for (int km = kdef; km >= kdef - 2 && km >= 1; km--) {
         // kernel choices only differ when the pass split does
