@@ -41,6 +41,32 @@ bool build_p2_params(const HasherSpec &h, P2Params<F, W> *p) {
                                h.out, p);
 }
 
+// One state a thread: the throughput form of instances that the tensor-core kernels are not built for (other
+// numbers of rounds).
+template <class F, int W>
+__global__ void __launch_bounds__(128)
+    states_kernel(typename F::T *__restrict__ states, size_t n, const __grid_constant__ P2Params<F, W> p) {
+  using T = typename F::T;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    T s[W];
+    T *g = states + i * W;
+#pragma unroll
+    for (int k = 0; k < W; k++) s[k] = Dom<F>::enter(g[k]);
+    p2_permute<F, W>(s, p);
+#pragma unroll
+    for (int k = 0; k < W; k++) g[k] = Dom<F>::leave(s[k]);
+  }
+}
+
+// States from which it beats quads of threads, whose permutations take a quarter more instructions.  BabyBear
+// 8 + 22 rounds: 19,000 states 22.5 us against 23.5, 40,000 29.7 against 33.8, 2^20 382 against 611; 8 + 14: equal up to
+// 28,000, 2^20 331 against 488.  Goldilocks 8 + 21: 60,000 169 against 155, 70,000 169 against 175, 2^20 1957 against
+// 2403.
+template <class F>
+static constexpr size_t one_per_thread() {
+  return sizeof(typename F::T) == 4 ? 148 * 128 + 1 : 1 << 16;
+}
+
 template <class F, int W>
 int p2_permute_batch(typename F::T *d_states, size_t n_states, const P2Params<F, W> &p,
                      cudaStream_t s) {
@@ -52,6 +78,13 @@ int p2_permute_batch(typename F::T *d_states, size_t n_states, const P2Params<F,
       return p2g::permute<W>(d_states, n_states, p, s);
   }
   const unsigned threads = 128;
+  if (n_states >= one_per_thread<F>()) {
+    DeviceContext *ctx;
+    ZKB_TRY(current_context(&ctx));
+    const unsigned grid = grid_for(n_states, threads, (unsigned)ctx->sm_count * 16u);
+    ZKB_LAUNCH("p2_permute", s, states_kernel<F, W><<<grid, threads, 0, s>>>(d_states, n_states, p));
+    return ZKB_OK;
+  }
   ZKB_LAUNCH("p2_permute", s, quad::states_kernel<F, W><<<quad::grid_of(n_states, threads), threads, 0, s>>>(d_states, n_states, p));
   ZKB_CHECK_LAUNCH();
   return ZKB_OK;
