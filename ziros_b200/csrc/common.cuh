@@ -124,8 +124,10 @@ struct ScratchBuf {
   ScratchBuf() = default;
   ScratchBuf(const ScratchBuf &) = delete;
   ScratchBuf &operator=(const ScratchBuf &) = delete;
-  ~ScratchBuf() {
+  ~ScratchBuf() { release(); }
+  void release() {
     if (p) dev_free(p, s);
+    p = nullptr;
   }
   int alloc(size_t bytes, cudaStream_t stream) {
     s = stream;

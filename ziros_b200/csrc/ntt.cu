@@ -821,13 +821,25 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
   const bool apart = (uintptr_t)(d_trace + n * stride) <= (uintptr_t)d_out ||
                      (uintptr_t)(d_out + (n << log_b) * stride) <= (uintptr_t)d_trace;
   const int kmax = tn.kmax ? tn.kmax : apart ? plan_kmax<F>(d_trace, n, width, stride) : pass_kmax<F>();
+  const std::vector<int> ks = plan_passes(log_h, kmax);
   // Natural order: the transform goes to scratch, its rows then into the caller's buffer, which holds the
-  // coefficients until then (the fused kernel has read them all), so that one scratch buffer is enough.
+  // coefficients until then (the fused kernel has read them all), so that one scratch buffer is enough.  Where
+  // that buffer cannot hold them (it overlaps the trace, or is not aligned for the tile copies) they have
+  // scratch of their own, or without room for both the transform runs in the caller's buffer and goes through
+  // the one scratch buffer afterwards.
   T *const natural = d_out;
-  ScratchBuf reversed;
+  ScratchBuf reversed, coef;
+  bool through = false;
   if (!bitrev) {
-    ZKB_TRY(reversed.alloc((n << log_b) * width * sizeof(T), s));
-    d_out = reversed.as<T>();
+    const bool own_coef = ks.size() > 1 && !coef_scratch && !(apart && ((uintptr_t)natural & 15) == 0);
+    int rc = own_coef ? coef.alloc(n * width * sizeof(T), s) : ZKB_OK;
+    if (rc == ZKB_OK) rc = reversed.alloc((n << log_b) * width * sizeof(T), s);
+    through = own_coef && rc == ZKB_ERR_OOM;
+    if (through)
+      clear_error();
+    else
+      ZKB_TRY(rc);
+    if (!through) d_out = reversed.as<T>();
   }
   const T *ctab;
   ZKB_TRY(get_coset_table<F>(log_h, log_b, shift, &ctab, s));
@@ -838,15 +850,13 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
     const T *itw, *ftw;
     ZKB_TRY(get_twiddles<F>(log_h, true, &itw, s));
     ZKB_TRY(get_twiddles<F>(log_h, false, &ftw, s));
-    const std::vector<int> ks = plan_passes(log_h, kmax);
     const int Kf = ks.back();
-    ScratchBuf coef;
     const T *src = d_trace;
     if (ks.size() > 1) {
       T *cs = coef_scratch;
       if (!cs && !bitrev && apart && ((uintptr_t)natural & 15) == 0) cs = natural;
       if (!cs) {
-        ZKB_TRY(coef.alloc(n * width * sizeof(T), s));
+        if (!coef.p) ZKB_TRY(coef.alloc(n * width * sizeof(T), s));
         cs = coef.as<T>();
       }
       std::vector<int> head(ks.begin(), ks.end() - 1);
@@ -895,6 +905,13 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
     if (!tail.empty())
       ZKB_TRY(run_plan<F>(d_out, d_out, log_h, width, 1ull << log_b, ftw, false, (T)0, tail,
                           log_h - Kf, s, tn.c_pass, stride));
+  }
+  if (through) {
+    coef.release();
+    ZKB_TRY(reversed.alloc((n << log_b) * width * sizeof(T), s));
+    ZKB_TRY(bitrev_rows<F>(natural, reversed.as<T>(), log_h + log_b, width, s));
+    ZKB_CHECK_CUDA(cudaMemcpyAsync(natural, reversed.p, (n << log_b) * width * sizeof(T), cudaMemcpyDeviceToDevice, s));
+    return ZKB_OK;
   }
   if (!bitrev) return bitrev_rows<F>(d_out, natural, log_h + log_b, width, s);
   return ZKB_OK;
