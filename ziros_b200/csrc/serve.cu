@@ -275,20 +275,22 @@ int zkb_engine_submit(zkb_engine *e, const zkb_job_desc *desc, uint64_t *job_id)
   ZKB_REQUIRE(!desc->with_fri || desc->hasher.field == ZKB_FIELD_BABYBEAR,
               "the FRI job runs over the BabyBear quartic extension");
   job->mem_estimate = job_bytes(*desc);
+  bool admissible;
   {
     std::lock_guard<std::mutex> lk(e->mu);
     ZKB_REQUIRE(job->mem_estimate <= e->budget,
                 "job needs ~%llu bytes of device memory, more than the engine budget %llu",
                 (unsigned long long)job->mem_estimate, (unsigned long long)e->budget);
     job->id = e->next_id++;
+    job->t_submit = Clock::now();
     (void)log_epoch();  // the job log's clock starts at the first submission
     e->jobs[job->id] = job;
     e->queue.push_back(job);
-    // Woken workers wait for the lock, so the time is taken before any of them sees the job, and
-    // waking them (system calls) does not lie between it and the return to the caller.
-    e->cv_queue.notify_all();
-    job->t_submit = Clock::now();
+    admissible = e->pick() != e->queue.end();
   }
+  // A job that no worker could admit now wakes none (the end of a job that frees memory does): its
+  // submission ends without their system calls.
+  if (admissible) e->cv_queue.notify_all();
   *job_id = job->id;
   return ZKB_OK;
 }
