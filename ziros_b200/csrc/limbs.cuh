@@ -6,11 +6,13 @@
 namespace zkb {
 namespace limbs {
 
+// Largest half of a BabyBear output's accumulators that `babybear` takes.
+constexpr uint64_t BABYBEAR_MAX_HALF = (uint64_t)BabyBear::P * 97 / 100;
 #ifdef __CUDACC__
-// BabyBear: a word congruent to a0 + a1 2^8 + a2 2^16 + a3 2^24 mod p, in [-p, 1.04 p]: u = a0 + a1 2^8 and
-// v = a2 + a3 2^8 stay below 0.97 p (at most 120 operand bytes, 120 * 255 * 255 * 257 < 2^31);
-// q = floor(v * 139810 / 2^32) is at most the true quotient of v 2^16 by p (2^32 * 2^16 / p = 139810.13) and
-// less than 1.07 below it.
+// BabyBear: a word congruent to a0 + a1 2^8 + a2 2^16 + a3 2^24 mod p, in [-p, 1.04 p], for u = a0 + a1 2^8 and
+// v = a2 + a3 2^8 of at most BABYBEAR_MAX_HALF: q = floor(v * 139810 / 2^32) is at most the true quotient of
+// v 2^16 by p (2^32 * 2^16 / p = 139810.13) and less than 1.07 below it, so v 2^16 - (q + 1) p lies in
+// [-p, 0.07 p].
 __device__ __forceinline__ int babybear(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
   const uint32_t u = a0 + (a1 << 8), v = a2 + (a3 << 8);
   const uint32_t q = __umulhi(v, 139810u) + 1;

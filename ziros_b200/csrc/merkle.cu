@@ -181,10 +181,9 @@ static int build_tree_impl(const HasherSpec &h, const std::vector<TreeMatrix> &m
   MatList ml;
   ZKB_TRY(make_list(0, ng, &ml));
   const unsigned thr = 128;
-  // One row (or pair) per thread and as many blocks as that takes: blocks retire every few
-  // milliseconds, so kernels of other streams (other jobs of the engine, which gives small
-  // jobs higher stream priority) get SMs in between instead of waiting for the whole grid.
-  (void)ctx;
+  // Both forms' blocks retire every few milliseconds at most (a quad's after a row or two, the tensor-core
+  // form's after a unit of work, p2_tensor.cu: shape), so kernels of other streams (other jobs of the
+  // engine, which gives small jobs higher stream priority) get SMs in between.
   // Leaf digests of the matrices in `l` (rows of one height).
   constexpr bool bb = std::is_same<F, BabyBear>::value;
   auto hash = [&](const MatList &l, uint64_t height, T *out, const LeafCombine *c, const char *name) -> int {

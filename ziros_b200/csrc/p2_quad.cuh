@@ -8,7 +8,7 @@
 // does.  Eight permutations a warp take about 2300 instructions, a quarter more than the same eight
 // in single lanes, so the form is also the one for middle sizes.
 //
-// Tree levels below that size are one launch for up to nine levels: a block takes a run of S nodes
+// Tree levels below that size are one launch for up to eight levels: a block takes a run of S nodes
 // and computes the whole subtree above them, level by level in shared memory.
 #pragma once
 #include "common.cuh"
@@ -420,7 +420,7 @@ __device__ __forceinline__ void subtree(uint64_t block, int levels, Layer layer,
   }
 }
 
-constexpr int MAX_RUN = 9;  // levels of one launch
+constexpr int MAX_RUN = 8;  // levels of one launch
 
 // Where a tree's layers lie: layer j of the run starts `off[j]` digests into `layers` and has n[j]
 // computed nodes.
@@ -506,13 +506,13 @@ __global__ void __launch_bounds__(128)
 
 inline unsigned grid_of(uint64_t items, unsigned threads) { return grid_for(items * 4, threads, 1u << 30); }
 
-// Levels per launch for a run of `total` levels: as few launches as MAX_RUN - 1 levels each allow, of
+// Levels per launch for a run of `total` levels: as few launches as MAX_RUN levels each allow, of
 // equal length.
 inline int run_levels(int total) {
-  const int stages = (total + MAX_RUN - 2) / (MAX_RUN - 1);
+  const int stages = (total + MAX_RUN - 1) / MAX_RUN;
   return (total + stages - 1) / stages;
 }
-// Four threads for each of the first level's nodes, and sixteen for each of its fourth's.
+// Four threads for each of the first level's nodes (up to 512), which is sixteen for each of the third's.
 inline unsigned run_threads(int levels) {
   const int t = 4 << (levels - 1);
   return (unsigned)(t < 32 ? 32 : t > 512 ? 512 : t);

@@ -218,6 +218,38 @@ constexpr bool absorb_fits() {
 }
 static_assert(absorb_fits(), "the fused absorb layer needs entries below 256");
 
+// The largest a0 + a1 2^8 or a2 + a3 2^8 that any output of a layer recombined by limbs::babybear can have:
+// operand bytes of 255 throughout, and the largest constant (0.489 p).
+constexpr uint64_t max_half() {
+  const Image m = make_image();
+  struct Part {
+    int base, N, steps, col0;  // matrix rows of accumulator columns col0 .. col0 + N
+  };
+  // the products that add up in one accumulator
+  const Part layers[6][3] = {{{I_IN16, 64, 2, 0}},
+                             {{I_ABS, 64, 3, 0}},  // every absorb matrix in turn, below
+                             {{I_Y, 64, 2, 0}, {I_B2, 48, 1, 16}, {I_B3, 32, 1, 32}},
+                             {{I_O, 64, 4, 0}},
+                             {{I_FIN8, 32, 2, 0}},
+                             {{I_FIN16, 64, 2, 0}}};
+  uint64_t best = 0;
+  for (int layer = 0; layer < 6; layer++)
+    for (int a = 0; a < (layer == 1 ? 8 : 1); a++) {
+      uint64_t sum[64] = {};
+      for (const Part &p : layers[layer])
+        for (int n = 0; n < p.N; n++)
+          for (int k = 0; k < 32 * p.steps; k++)
+            sum[p.col0 + n] += m.b[p.base + a * ABS_BYTES + (k / 32) * p.N * 32 + slot(p.N, n, k % 32)];
+      for (int i = 0; i < 16; i++)
+        for (int h = 0; h < 4; h += 2) {
+          const uint64_t v = 255 * (sum[4 * i + acc_col(h)] + 256 * sum[4 * i + acc_col(h + 1)]) + 65535;
+          best = v > best ? v : best;
+        }
+    }
+  return best;
+}
+static_assert(max_half() <= limbs::BABYBEAR_MAX_HALF, "accumulators exceed the recombination's range");
+
 #ifdef __CUDACC__
 static __device__ constexpr Coefs kCoefs = make_coefs();
 static __device__ const Image kImage = make_image();
@@ -274,8 +306,9 @@ __device__ __forceinline__ int smul2(int a0, int b0, int a1, int b1) {
   const int m = (int)((uint32_t)t * BabyBear::PINV);
   return (int)(t >> 32) - __mulhi(m, (int)P);
 }
-// x^7 of any int32 input, in (-p, p): |x2| <= 2^30 + p/2, |x3| <= 2^30 + p/2, |x4| < p, so the last
-// product has |x3 x4| < 2^62 / 2.
+// x^7 of any int32 input, in (-p, p).  A product a b gives |a b| / 2^32 + p / 2 at most in absolute value:
+// 1.0334 p for x2, 1.0167 p for x3, 1.0006 p for x4, and the last product's |x3 x4| <= 1.0173 p^2 = 4.124e18 is
+// below the 2^31 p = 4.323e18 that keeps its result in (-p, p).
 __device__ __forceinline__ int sbox(int x) {
   const int x2 = smul(x, x);
   const int x3 = smul(x2, x);

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// States from which it beats quads of threads, whose permutations take a quarter more instructions.  BabyBear
+// States from which it beats quads of threads (p2_quad.cuh).  BabyBear
 // 8 + 22 rounds: 19,000 states 22.5 us against 23.5, 40,000 29.7 against 33.8, 2^20 382 against 611; 8 + 14: equal up to
 // 28,000, 2^20 331 against 488.  Goldilocks 8 + 21: 60,000 169 against 155, 70,000 169 against 175, 2^20 1957 against
 // 2403.
