@@ -93,3 +93,19 @@ def test_a_captured_plan_outlives_a_smaller_one():
     small.run()
     plan.run()
     assert (plan.roots() == want).all()
+
+
+@pytest.mark.parametrize("field,p2,log_h", [(Z.BABYBEAR, 16, 20), (Z.GOLDILOCKS, 12, 18)])
+def test_levels_of_fewer_trees_in_one_capture(field, p2, log_h):
+    """One tall trace among small ones: the small trees end while the tall one's levels still take the
+    tensor-core form, so one graph holds launches of many trees and of one."""
+    shapes = [(1 << log_h, 4)] + [(1 << 3, 4)] * 20
+    plan = Z.BatchCommit(shapes, field=field, p2_width=p2, autotune=False)
+    traces = [_uniform(field, s, i) for i, s in enumerate(shapes)]
+    for i, t in enumerate(traces):
+        plan.copy_in(i, t)
+    pcs = Z.CudaTwoAdicPcs(field, 42, 1, p2)
+    want = np.stack([pcs.commit_dev(t)[0] for t in traces])
+    for _ in range(2):
+        plan.run()
+        assert (plan.roots() == want).all()
