@@ -1,5 +1,6 @@
-"""Batch permutations with numbers of rounds that the tensor-core kernels are not built for: quads of
-threads below a size, one state a thread from there on."""
+"""Batch permutations by their form: quads of threads for few states, one state a thread for more and
+for numbers of rounds that the tensor-core kernels are not built for, the tensor-core kernel by the
+number of 128-state tiles an SM."""
 import numpy as np
 import pytest
 import torch
@@ -28,6 +29,12 @@ def test_equals_the_oracle(oracle, field, ext, internal, n):
     pick = np.unique(np.r_[0, n - 1, np.random.default_rng(n).integers(0, n, 1500)])
     want = np.asarray(oracle.permute(field, st[pick].copy(), rc, ext, internal)).reshape(-1, 16)
     assert (got[pick] == want).all()
+
+
+# the standard instance, around the sizes at which 148 SMs get one tile more
+@pytest.mark.parametrize("n", [18944, 18945, 37888, 37889, 94720, 94721, 246272, 246273])
+def test_tiles_per_sm(oracle, n):
+    test_equals_the_oracle(oracle, Z.BABYBEAR, 8, 13, n)
 
 
 def test_large_batches_do_not_run_as_quads():

@@ -41,8 +41,8 @@ bool build_p2_params(const HasherSpec &h, P2Params<F, W> *p) {
                                h.out, p);
 }
 
-// One state a thread: the throughput form of instances that the tensor-core kernels are not built for (other
-// numbers of rounds).
+// One state a thread: the form of middle sizes (tensor_batch below), and of large ones for instances that the
+// tensor-core kernels are not built for (other numbers of rounds).
 template <class F, int W>
 __global__ void __launch_bounds__(128)
     states_kernel(typename F::T *__restrict__ states, size_t n, const __grid_constant__ P2Params<F, W> p) {
@@ -67,26 +67,38 @@ static constexpr size_t one_per_thread() {
   return sizeof(typename F::T) == 4 ? 148 * 128 + 1 : 1 << 16;
 }
 
+// The tensor-core form of a batch: one permutation a state, so its tables and a last round of fewer than five
+// tiles an SM are not paid for as a leaf hash's are.  BabyBear by 128-state tiles an SM (148 SMs), against one
+// state a thread: two tiles 23.0 us against 21.0, three to five 25.0, 27.1 and 32.5 against 27.2, 27.2 and 33.0, six
+// to thirteen slower or equal (100,000 states 45.3 against 43.4, 200,000 70.7 against 68.2), from fourteen on
+// faster (400,000 122 against 128, 2^20 273 against 322).  Goldilocks is faster at every size.
+template <class F>
+static bool tensor_batch(size_t n, int sms) {
+  if (sizeof(typename F::T) == 8) return true;
+  const uint64_t tiles = ((n + 127) / 128 + sms - 1) / sms;
+  return (tiles >= 3 && tiles <= 5) || tiles >= 14;
+}
+
 template <class F, int W>
 int p2_permute_batch(typename F::T *d_states, size_t n_states, const P2Params<F, W> &p,
                      cudaStream_t s) {
   if (n_states == 0) return ZKB_OK;
-  if (tensor_takes<F, W>(p, n_states)) {
-    if constexpr (std::is_same<F, BabyBear>::value)
-      return p2t::permute(d_states, n_states, p, s);
-    else
-      return p2g::permute<W>(d_states, n_states, p, s);
-  }
   const unsigned threads = 128;
-  if (n_states >= one_per_thread<F>()) {
+  const bool tensor = tensor_takes<F, W>(p, n_states);
+  if (tensor || n_states >= one_per_thread<F>()) {
     DeviceContext *ctx;
     ZKB_TRY(current_context(&ctx));
+    if (tensor && tensor_batch<F>(n_states, ctx->sm_count)) {
+      if constexpr (std::is_same<F, BabyBear>::value)
+        return p2t::permute(d_states, n_states, p, s);
+      else
+        return p2g::permute<W>(d_states, n_states, p, s);
+    }
     const unsigned grid = grid_for(n_states, threads, (unsigned)ctx->sm_count * 16u);
     ZKB_LAUNCH("p2_permute", s, states_kernel<F, W><<<grid, threads, 0, s>>>(d_states, n_states, p));
     return ZKB_OK;
   }
   ZKB_LAUNCH("p2_permute", s, quad::states_kernel<F, W><<<quad::grid_of(n_states, threads), threads, 0, s>>>(d_states, n_states, p));
-  ZKB_CHECK_LAUNCH();
   return ZKB_OK;
 }
 
