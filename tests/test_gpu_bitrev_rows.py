@@ -1,4 +1,5 @@
-"""The row permutation behind the natural-order transforms: blocks of 32 to 1,024 rows by the width."""
+"""The row permutation behind the natural-order transforms: rows per block by the width and the height,
+and rows written in runs of eight where single ones would share their sectors."""
 import ctypes as C
 
 import numpy as np
@@ -29,13 +30,33 @@ def test_transforms_in_natural_order(oracle, field, width):
     assert (lde[order] == rev).all()
 
 
-def _permutation_us(log_h, width):
+# runs from 48 MB on for rows that are not whole sectors: both sides of the line in bytes and in the width
+@pytest.mark.parametrize("field,log_n,width", [
+    (Z.BABYBEAR, 20, 1), (Z.BABYBEAR, 19, 3), (Z.BABYBEAR, 20, 11), (Z.BABYBEAR, 20, 12), (Z.BABYBEAR, 20, 16), (Z.BABYBEAR, 21, 8),
+    (Z.BABYBEAR, 18, 63), (Z.BABYBEAR, 18, 64), (Z.BABYBEAR, 18, 65), (Z.GOLDILOCKS, 19, 2), (Z.GOLDILOCKS, 20, 5),
+    (Z.GOLDILOCKS, 20, 6), (Z.GOLDILOCKS, 18, 32), (Z.GOLDILOCKS, 18, 33), (Z.GOLDILOCKS, 17, 63), (Z.GOLDILOCKS, 17, 65)])
+def test_natural_order_is_the_bit_reversed_one_permuted(field, log_n, width):
+    dft = Z.CudaDft(field)
+    dt = torch.int32 if field == Z.BABYBEAR else torch.int64
+    x = torch.randint(0, 0x78000001, (1 << (log_n - 1), width), dtype=dt, device="cuda")
+    nat, rev = (torch.empty((1 << log_n, width), dtype=dt, device="cuda") for _ in range(2))
+    dft.coset_lde_batch_dev(x, 1, nat, bit_reverse_rows=False)
+    dft.coset_lde_batch_dev(x, 1, rev)
+    i = torch.arange(1 << log_n, device="cuda")
+    order = torch.zeros_like(i)
+    for b in range(log_n):
+        order |= ((i >> b) & 1) << (log_n - 1 - b)
+    assert torch.equal(nat[order], rev)
+
+
+def _permutation_us(log_h, width, field=Z.BABYBEAR):
     lib = N.load()
-    x = torch.randint(0, 0x78000001, (1 << log_h, width), dtype=torch.int32, device="cuda")
+    dt = torch.int32 if field == Z.BABYBEAR else torch.int64
+    x = torch.randint(0, 0x78000001, (1 << log_h, width), dtype=dt, device="cuda")
     stats = (N.KernelStat * 64)()
 
     def transform():
-        N.check(lib.zkb_dft_batch_dev(Z.BABYBEAR, C.c_void_p(x.data_ptr()), log_h, width, 0, None))
+        N.check(lib.zkb_dft_batch_dev(field, C.c_void_p(x.data_ptr()), log_h, width, 0, None))
 
     transform()
     lib.zkb_profile_start()
@@ -48,6 +69,12 @@ def _permutation_us(log_h, width):
 
 
 def test_a_narrow_matrix_takes_no_more_blocks_than_a_wide_one():
-    """2^22 words as one column against sixteen: the writes of single words cost about twice as much
-    (29 us and 14 on a B200); blocks that are mostly idle would make it five times."""
+    """2^22 words as one column against sixteen (16 us and 12 on a B200); blocks that are mostly idle
+    would make it five times."""
     assert _permutation_us(22, 1) < 3.5 * _permutation_us(18, 16)
+
+
+def test_rows_of_partial_sectors_are_written_together():
+    """2^21 x 9 Goldilocks words (72-byte rows) against 2^21 x 8: rows written one at a time would read and
+    write their shared sectors again, 2.6 times as long."""
+    assert _permutation_us(21, 9, Z.GOLDILOCKS) < 1.8 * _permutation_us(21, 8, Z.GOLDILOCKS)

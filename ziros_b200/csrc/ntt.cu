@@ -680,35 +680,60 @@ static int launch_fused(const typename F::T *in, typename F::T *out, const Fused
 }
 
 // ------------------------------------------------------- auxiliary kernels
-// out[rev(row)] = in[row].  A block takes 2^lr consecutive rows, read as one run of elements whose rows
-// come from 32-bit divisions; bound by the writes, runs of one row each.  Blocks of at least 32 rows and
-// 1,024 elements, four a thread: with 32 rows whatever the width, 2^22 x 1 words take 74 us (29 now), 2^20 x 4
-// 22.9 (12.6), 2^20 x 16 53 (34); 512 elements 2^20 x 8 22.8 (16.8), 4,096 2^16 x 1 10 (6.5).  2^18 x 37:
-// 19.5 us; runs of eight rows on both sides, fewer elements in flight per thread, 39.
-constexpr int BITREV_MIN_LOG = 5, BITREV_MAX_LOG = 10;
-constexpr uint64_t BITREV_ELEMS = 1024;
-template <class F, class Idx>
+// out[rev(row)] = in[row], 2^lr rows a block, elements dealt out by 32-bit divisions.
+//
+// RUNS = false: consecutive rows, read as one run and written a row at a time.  Bound by the writes.
+// RUNS = true: 2^(lr - 3) consecutive rows in each of eight places N / 8 apart, so that eight rows at a time are
+// written side by side.  A row that does not fill its 32-byte sectors shares them with rows N / 2 away;
+// in a matrix larger than L2 those would be written long after, each time a sector read and written again.
+constexpr int RUN_LOG = 3;
+template <class F, class Idx, bool RUNS>
 __global__ void __launch_bounds__(256) bitrev_rows_kernel(const typename F::T *__restrict__ in,
                                                           typename F::T *__restrict__ out, int L, uint32_t width, int lr) {
-  const uint64_t row0 = (uint64_t)blockIdx.x << lr, left = (1ull << L) - row0;
-  const Idx n = (Idx)(left < (1ull << lr) ? left : 1ull << lr) * width;
-  const typename F::T *src = in + row0 * width;
+  const Idx n = (Idx)width << lr;
+  if constexpr (RUNS) {
+    const uint64_t p0 = (uint64_t)blockIdx.x << (lr - RUN_LOG);
+    const int rest = L - RUN_LOG;
+    const Idx run = (Idx)width << RUN_LOG;
 #pragma unroll 4
-  for (Idx e = threadIdx.x; e < n; e += 256) {
-    const Idx r = e / width, c = e - r * width;
-    const uint64_t to = L ? (__brevll(row0 + r) >> (64 - L)) : 0;
-    out[to * width + c] = src[e];
+    for (Idx e = threadIdx.x; e < n; e += 256) {
+      const Idx p = e / run, x = e - p * run, q = x / width, c = x - q * width;
+      const uint64_t from = ((uint64_t)(__brev((uint32_t)q) >> (32 - RUN_LOG)) << rest) + p0 + p;
+      const uint64_t to = ((rest ? __brevll(p0 + p) >> (64 - rest) : 0) << RUN_LOG) + q;
+      out[to * width + c] = in[from * width + c];
+    }
+  } else {
+    const uint64_t row0 = (uint64_t)blockIdx.x << lr;
+    const typename F::T *src = in + row0 * width;
+#pragma unroll 4
+    for (Idx e = threadIdx.x; e < n; e += 256) {
+      const Idx r = e / width, c = e - r * width;
+      const uint64_t to = L ? (__brevll(row0 + r) >> (64 - L)) : 0;
+      out[to * width + c] = src[e];
+    }
   }
 }
+// Runs for rows of at most three elements, and from 48 MB on for rows that are not whole sectors (or one):
+// 2^22 x 1 words 15.5 us against 29 (2^20 x 3 12.7 against 13.8), 2^21 x 9 words 48 against 80, 2^20 x 37 86 against 129, 2^22 x 8
+// 74 against 113, but 2^20 x 10 (42 MB) 29 against 23 and 2^20 x 16 (two sectors) 41 against 35; Goldilocks 2^21 x 9 59 against
+// 185, 2^20 x 12 38 against 50, and equal from 256-byte rows on.
+// A block has at least 256 elements, and more up to 8 KB (16 KB of runs) once there are eight blocks an SM: 2^8 x 256
+// words in blocks of 32 rows took 8.6 us (6.5), 2^22 x 1 in blocks of 32 elements 74 us.
 template <class F>
 static int bitrev_rows(const typename F::T *in, typename F::T *out, int L, uint32_t width, cudaStream_t s) {
-  int lr = BITREV_MIN_LOG;
-  while (lr < BITREV_MAX_LOG && ((uint64_t)width << lr) < BITREV_ELEMS) lr++;
-  const unsigned blocks = (unsigned)(((1ull << L) + (1ull << lr) - 1) >> lr);
-  if (width < (1u << 26))
-    ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F, uint32_t><<<blocks, 256, 0, s>>>(in, out, L, width, lr));
+  const uint64_t row = (uint64_t)width * sizeof(typename F::T), total = row << L;
+  const bool sectors = sizeof(typename F::T) == 4 ? row >= 256 || (row > 32 && row % 32 == 0) : row >= 512 || row % 256 == 0;
+  const bool runs = L >= RUN_LOG && (width <= 3 || (total >= 48ull << 20 && !sectors));
+  int lr = runs ? RUN_LOG : 0;
+  while (lr < L && ((uint64_t)width << lr) < 256) lr++;
+  while (lr < L && (1ull << (L - lr)) > 8 * 148 && row << lr < (runs ? 16384u : 8192u)) lr++;
+  const unsigned blocks = (unsigned)(1ull << (L - lr));
+  if (runs)
+    ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F, uint32_t, true><<<blocks, 256, 0, s>>>(in, out, L, width, lr));
+  else if (width < (1u << 26))
+    ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F, uint32_t, false><<<blocks, 256, 0, s>>>(in, out, L, width, lr));
   else
-    ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F, uint64_t><<<blocks, 256, 0, s>>>(in, out, L, width, lr));
+    ZKB_LAUNCH("bitrev_rows", s, bitrev_rows_kernel<F, uint64_t, false><<<blocks, 256, 0, s>>>(in, out, L, width, lr));
   return ZKB_OK;
 }
 
