@@ -477,9 +477,15 @@ static constexpr int pass_kmax() {
   return sizeof(typename F::T) == 4 ? 10 : 7;
 }
 
-// Smallest Goldilocks pass (in tiles) on the tensor cores: nearly one tile an SM.  2^16 x 30: 100 us with them
-// from 300 tiles on, 142 from 1,480 on; 2^16 x 8 45 from 140 on, 57 from 296 on.
-static constexpr uint64_t NTT_TC_MIN_TILES = 128;
+// Smallest Goldilocks pass and fused middle (in tiles) on the tensor cores.  A block sets up tables and TMEM (a
+// pass takes at least 10.5 us, as butterflies 8.5), so the fewer index bits the more tiles make up for it.  Passes
+// of 6 bits: 1,536 tiles 19.4 us against 18.9, 2,048 20.9 against 23.0 (128: 10.5 against 8.7); of 7: 128 tiles 12.8
+// against 12.2, 256 equal, 512 15.3 against 17.9; of 8, nearly one tile an SM: with them a plan needs a pass less
+// (2^16 x 8 25.6 us against 33.1).  Fused middle, blowup 2: 6 bits 128 tiles 14.6 against 13.3, 256 equal, 384 16.8 against
+// 18.5; 7 bits 128 tiles 19.0 against 22.9.
+static constexpr uint64_t tc_min_tiles(int K, bool fused) {
+  return K == 6 ? (fused ? 384 : 2048) : K == 7 && !fused ? 256 : 128;
+}
 
 // Largest pass of a default plan over n rows of `width` columns: a Goldilocks pass of 8 bits is slower than
 // one of 7 as butterflies and faster on the tensor cores (2^16 x 30: two passes, 100 us, against
@@ -488,7 +494,7 @@ template <class F>
 static int plan_kmax(const void *base, uint64_t n, uint32_t width, uint32_t stride) {
   if constexpr (sizeof(typename F::T) == 8) {
     const uint32_t C = ntt_tc::chunk(8), chunks = (width + C - 1) / C;
-    if (n >= 256 && chunks * (n >> 8) >= NTT_TC_MIN_TILES && (chunks * C - width) * 4 <= width &&
+    if (n >= 256 && chunks * (n >> 8) >= tc_min_tiles(8, false) && (chunks * C - width) * 4 <= width &&
         ntt_tile_loads().load() == 1 && stride % 2 == 0 && ((uintptr_t)base & 15) == 0)
       return 8;
   }
@@ -530,7 +536,7 @@ static int run_plan(const typename F::T *in, typename F::T *out, int L, uint32_t
       const uint32_t C = tc ? ntt_tc::chunk(K) : 0;
       const uint32_t chunks = C ? (width + C - 1) / C : 0;
       const uint64_t tiles = (uint64_t)chunks * g.groups * n_blocks;
-      if (C && tiles >= NTT_TC_MIN_TILES && (chunks * C - width) * 4 <= width &&
+      if (C && tiles >= tc_min_tiles(K, false) && (chunks * C - width) * 4 <= width &&
           tma_tiles(src, sizeof(T), stride, C, L, g.lo, K, n_blocks, width)) {
         CUtensorMap map;
         ZKB_TRY(pass_tensor_map(&map, src, sizeof(T), g, width, K, n_blocks, C));
@@ -901,7 +907,7 @@ int ntt_lde_dev(const typename F::T *d_trace, int log_h, uint32_t width, int log
       const uint32_t C = tn.c_fused ? 0 : ntt_tc::chunk(Kf);
       const uint32_t chunks = C ? (width + C - 1) / C : 0;
       const uint64_t tiles = (uint64_t)chunks * g.blocks;
-      if (C && tiles >= NTT_TC_MIN_TILES && (chunks * C - width) * 4 <= width &&
+      if (C && tiles >= tc_min_tiles(Kf, true) && (chunks * C - width) * 4 <= width &&
           tma_tiles(src, sizeof(T), stride, C, log_h, 0, Kf, 1, width)) {
         // block B's rows as the tile of a pass at bits [0, K) of one transform
         PassGeom pg;
