@@ -78,11 +78,8 @@ int take_wait_errors(uint32_t *count);  // since the last call; acknowledges the
 // complete takes 4 us (a product or a tile copy takes a few; the limit is for what never comes).
 constexpr uint32_t WAIT_POLLS = 1u << 24;
 #ifdef __CUDACC__
-// No fence: the end of the kernel makes it visible to a host that has waited for it.  Out of line, as the
-// other code that runs only when a wait has given up (tcgen05.cuh): inlined into each of a hashing kernel's
-// layers it costs 1 to 4 % (leaf hash with the alpha-reduction 2^21 x 256 17.07 ms against 16.64, Goldilocks
-// width-16 2^20 x 64 10.04 against 9.62).
-static __device__ __noinline__ void report_wait(uint32_t *word) { atomicAdd(word, 1u); }
+// No fence: the end of the kernel makes it visible to a host that has waited for it.
+__device__ __forceinline__ void report_wait(uint32_t *word) { atomicAdd(word, 1u); }
 #endif
 // Stream of the calling thread on its current device (created on first use).
 cudaStream_t thread_stream();

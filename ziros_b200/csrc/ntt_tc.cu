@@ -122,7 +122,6 @@ __device__ __forceinline__ void group_wait(Group &g, uint32_t mbar, uint32_t &ph
   if (wait_parity(mbar, phase, g.polls)) {
     phase ^= 1;
   } else {
-    if (g.polls) report_wait(g.err);
     g.polls = 0;
     if (in_flight) wait_parity(mbar, phase, WAIT_POLLS);
   }

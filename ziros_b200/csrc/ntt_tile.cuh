@@ -178,7 +178,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
 // block may end with its copy under way.  (A second wait after the first, or one at the block's end, cost the
 // passes up to 4 % and 2 %: BabyBear 2^22 x 256 13.1 ms against 12.7, 2^20 x 64 482 us against 467.)
 __device__ __forceinline__ void tile_wait(uint64_t *bar, uint32_t *err) {
-  if (!mbar_wait(bar, 0, 2 * WAIT_POLLS)) atomicAdd(err, 1u);
+  if (!mbar_wait(bar, 0, 2 * WAIT_POLLS)) report_wait(err);
 }
 
 __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, uint64_t *bar, int c0, int c1, int c2,

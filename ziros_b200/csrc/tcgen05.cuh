@@ -143,42 +143,38 @@ __device__ __forceinline__ void commit(uint32_t mbar, uint32_t one) {
       "r"(one)
       : "memory");
 }
-// After the lead warp has issued the products: everyone waits for them (bounded: a wait that runs
-// out reports itself and the group goes on without waiting, so every block ends).
+// After the lead warp has issued the products: everyone waits for them (bounded: a thread whose wait runs
+// out goes on without waiting, so every block ends, and reports it there, see drain: the report at every wait
+// made the hashing kernels 1 to 4 % longer, as a call 3 % that of column slabs).
 __device__ __forceinline__ void finish(Group &g) {
   if (g.lead) commit(g.mbar, g.one);
-  if (!wait_parity(g.mbar, g.phase, g.polls)) {
-    if (g.polls) report_wait(g.err);
-    g.polls = 0;
-  }
+  if (!wait_parity(g.mbar, g.phase, g.polls)) g.polls = 0;
   g.phase ^= 1;
   fence_after();
 }
-// Before the block gives its TMEM and shared memory back: where a wait gave up, products may still be under
-// way, so the lane that issued them waits for all of them on an mbarrier of its own (bounded), in the first
-// words of the tables, which nothing correct needs any more.
-static __device__ __noinline__ void drain_on(uint32_t mbar, uint32_t polls) {
+// Before the block gives its TMEM and shared memory back: a thread whose wait gave up reports it, and as products
+// may still be under way then, the lane that issued them waits for all of them on an mbarrier of its own
+// (bounded), in the first words of the tables, which nothing correct needs any more.
+__device__ __forceinline__ void drain(const Group &g, uint32_t polls = WAIT_POLLS) {
+  if (g.polls) return;
+  report_wait(g.err);
+  if (!g.one) return;
+  const uint32_t mbar = g.sm + 8 * (g.bar - 1);
   init_barrier(mbar);
   init_fence();
   commit(mbar, 1);
   wait_parity(mbar, 0, polls);
 }
-__device__ __forceinline__ void drain(const Group &g, uint32_t polls = WAIT_POLLS) {
-  if (!g.polls && g.one) drain_on(g.sm + 8 * (g.bar - 1), polls);
-}
 // The tables' copies (on the mbarrier `tables`) have landed; or they have not within the limit, and the
 // block reports that, waits once more, frees its TMEM (address at `slot`) and ends.  Every thread calls it.
-static __device__ __noinline__ void exit_without_tables(uint32_t tables, const uint8_t *slot, uint32_t cols,
-                                                        uint32_t *err, uint32_t polls) {
+__device__ __forceinline__ void tables_or_exit(uint32_t tables, const uint8_t *slot, uint32_t cols, uint32_t *err,
+                                               uint32_t polls = WAIT_POLLS) {
+  if (__syncthreads_and(wait_parity(tables, 0, polls))) return;
   if (threadIdx.x == 0) report_wait(err);
   wait_parity(tables, 0, polls);
   __syncthreads();
   if (threadIdx.x < 32) tmem_free(*reinterpret_cast<const volatile uint32_t *>(slot), cols);
   asm volatile("exit;");
-}
-__device__ __forceinline__ void tables_or_exit(uint32_t tables, const uint8_t *slot, uint32_t cols, uint32_t *err,
-                                               uint32_t polls = WAIT_POLLS) {
-  if (!__syncthreads_and(wait_parity(tables, 0, polls))) exit_without_tables(tables, slot, cols, err, polls);
 }
 // This thread's group: `cols` TMEM columns each from the address at sm + slot on, mbarriers at
 // `mbars`, tables at `sm`.
