@@ -8,9 +8,9 @@
 //
 // What bounds them: the integer multiplier.  The 564 products of a permutation's S-boxes occupy
 // it for 5640 cycles per warp (a wide product 4, a low one 2, a high one 4), everything else for
-// 1270.  On a B200 at 1965 MHz a leaf hash of 2^23 x 256 with the alpha-reduction runs 4.34e9
-// permutations/s (61.9 ms; 78.2 with the layers as modular additions, p2_permute); of 2^20 x 64 the multiplier
-// is 82 % busy, the ALU 31 %, the tensor pipe 11 %.
+// 1270.  On a B200 at 1965 MHz a leaf hash of 2^23 x 256 with the alpha-reduction runs 4.30e9
+// permutations/s (62.5 ms; 78.2 with the layers as modular additions, p2_permute); of 2^20 x 64 the multiplier
+// is 79 % busy, the ALU 31 %, the tensor pipe 11 %.
 #include <algorithm>
 
 #include "common.cuh"

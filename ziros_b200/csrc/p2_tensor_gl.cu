@@ -3,9 +3,9 @@
 // the TMEM of an SM holds three tiles of width 12 (168 columns each) and two of width 16 (208).
 //
 // What bounds them: the latency of the chains of 64-bit products (472 in a permutation's S-boxes at width 12, 600
-// at 16), which three or two warps a scheduler cover in part: 2^18 x 64 rows keep the multiplier 63 and 55 %
-// busy, the ALU 60 and 53 %, the issue slots 55 and 48 %.  On a B200 at 1965 MHz a 2^20 x 64 leaf hash takes
-// 6.10 and 8.22 ms; with the layers as modular additions and the partial rounds' diagonal as products, one state
+// at 16), which three or two warps a scheduler cover in part: 2^18 x 64 rows keep the multiplier 62 and 53 %
+// busy, the ALU 60 and 51 %, the issue slots 54 and 46 %.  On a B200 at 1965 MHz a 2^20 x 64 leaf hash takes
+// 6.11 and 8.52 ms; with the layers as modular additions and the partial rounds' diagonal as products, one state
 // per thread, it took 11.63 and 15.18 ms.
 #include <algorithm>
 
